@@ -6,12 +6,14 @@ there is no fallback and importing this module raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 from pathlib import Path
 
 import torch
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "libflare_b200.so"
+OPS_PATH = PKG / "_flare_torch.so"
 
 F32, F16, BF16 = 0, 1, 2
 TERM_GATHER, TERM_SCATTER, TERM_BOTH = 1, 2, 3
@@ -98,6 +100,20 @@ lib = _load()
 
 class FlareError(RuntimeError):
     pass
+
+
+def _load_ops():
+    """The operators on top of the C ABI (csrc/binding): registers torch.ops.flare_b200.* and holds the direct calls."""
+    if not OPS_PATH.exists():
+        raise ImportError(f"{OPS_PATH} is missing: build it with `python {PKG / 'build.py'}`")
+    spec = importlib.util.spec_from_file_location("_flare_torch", OPS_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.set_error_type(FlareError)
+    return mod
+
+
+native = _load_ops()
 
 
 def check(rc: int, what: str) -> None:

@@ -1,4 +1,4 @@
-"""Builds libflare_b200.so (sm_100a) in-tree with nvcc.  No GPU is needed to build."""
+"""Builds libflare_b200.so (sm_100a, nvcc) and _flare_torch.so (its torch operators, g++) in-tree.  No GPU is needed."""
 from __future__ import annotations
 
 import hashlib
@@ -6,12 +6,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libflare_b200.so"
+BINDING_SRC = CSRC / "binding" / "flare_torch.cpp"
+BINDING = PKG / "_flare_torch.so"
 STAMP = PKG / "csrc" / ".build_stamp"
 
 NVCC_FLAGS = [
@@ -28,6 +31,23 @@ def _nvcc() -> str:
     return cand
 
 
+def _binding_cmd():
+    """The torch operators: host code only, linked against this torch and libflare_b200.so beside it."""
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [INCLUDE, root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+           sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[f"-I{d}" for d in inc], str(BINDING_SRC), "-o", str(BINDING), f"-L{PKG}", "-lflare_b200", "-Wl,-rpath,$ORIGIN",
+            f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+
+
+def _torch_version() -> str:
+    import torch
+    return torch.__version__
+
+
 def sources():
     return sorted(CSRC.glob("*.cu"))
 
@@ -35,17 +55,18 @@ def sources():
 def _digest() -> str:
     h = hashlib.sha256()
     for f in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
-                    + list(INCLUDE.glob("*.h"))):
+                    + list(INCLUDE.glob("*.h")) + [BINDING_SRC]):
         h.update(f.name.encode())
         h.update(f.read_bytes())
     h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(_torch_version().encode())
     return h.hexdigest()
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every .cu under csrc/ into one shared library; skip when sources are unchanged."""
+    """Compile every .cu under csrc/ into one shared library and the operators on top of it; skip when sources are unchanged."""
     dig = _digest()
-    if not force and LIB.exists() and STAMP.exists() and STAMP.read_text() == dig:
+    if not force and LIB.exists() and BINDING.exists() and STAMP.exists() and STAMP.read_text() == dig:
         return LIB
     objdir = PKG / "build"
     objdir.mkdir(exist_ok=True)
@@ -70,6 +91,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("link failed")
+    r = subprocess.run(_binding_cmd(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError(f"building {BINDING.name} failed")
     STAMP.write_text(dig)
     return LIB
 
