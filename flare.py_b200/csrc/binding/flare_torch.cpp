@@ -424,35 +424,68 @@ Tensor causal_decode(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
 
 class CausalFn : public torch::autograd::Function<CausalFn> {
  public:
-  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
     at::AutoDispatchBelowADInplaceOrView below;
-    Tensor y = std::get<0>(causal_prefill(q, k, v, scale, std::nullopt));
-    ctx->save_for_backward({q, k, v});
+    for (const Tensor* t : {&q_, &k_, &v_}) need_cuda(*t);
+    same_dtype("q, k, v must share a dtype", {&q_, &k_, &v_});
     ctx->saved_data["scale"] = scale;
+    c10::cuda::CUDAGuard guard(k_.device());
+    const Tensor q = latents(q_), k = tok(k_), v = tok(v_);
+    FlareProblem p = problem(q, k, scale);
+    // the tensor-core shapes keep the chunk-start states for the backward (M (2 D + 8) bytes per 128 tokens and head);
+    // the others rebuild them there
+    const size_t bytes = flare_causal_train_bytes(&p);
+    Tensor y, saved;
+    if (bytes) {
+      y = at::detail::empty_cuda(k.sizes(), k.options());
+      set_stride(p.v_stride, v);
+      set_stride(p.y_stride, y);
+      saved = scratch(bytes, k);
+      check_rc(flare_causal_train_fwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), y.data_ptr(), saved.data_ptr(), stream_of(k)),
+               "flare_causal_train_fwd");
+    } else {
+      y = std::get<0>(causal_prefill(q_, k_, v_, scale, std::nullopt));
+    }
+    ctx->save_for_backward({q_, k_, v_, saved});
     return y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
-    const Tensor& q_ = s[0];
+    const Tensor &q_ = s[0], &saved = s[3];
     c10::cuda::CUDAGuard guard(s[1].device());
     const Tensor q = latents(q_), k = tok(s[1]), v = tok(s[2]), dy = tok(g[0]);
     FlareProblem p = problem(q, k, ctx->saved_data["scale"].toDouble());
     Tensor dk = at::detail::empty_cuda(k.sizes(), k.options()), dv = at::detail::empty_cuda(v.sizes(), v.options());
-    Tensor dq = f32({p.B, p.H, p.M, p.D}, k);
     set_stride(p.v_stride, v);
     set_stride(p.dy_stride, dy);
     set_stride(p.dk_stride, dk);
     set_stride(p.dv_stride, dv);
-    const Tensor ws = scratch(flare_causal_bwd_workspace_bytes(&p), k);
     const flare_stream_t st = stream_of(k);
-    check_rc(flare_causal_bwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), dy.data_ptr(), fp(dq), dk.data_ptr(),
-                              dv.data_ptr(), fp(ws), st), "flare_causal_bwd");
-    // one latent gradient per (b, h): shared latents sum over the batch; a batch made by expand() gets the
-    // per-batch gradients, which autograd folds back itself
-    if (q_.dim() == 3) {
-      Tensor sum = f32({p.H, p.M, p.D}, k);
-      check_rc(flare_reduce_sum(fp(dq), p.B, (int64_t)p.H * p.M, p.D, fp(sum), st), "flare_reduce_sum");
-      dq = sum;
+    const bool shared = q_.dim() == 3;
+    Tensor dq;
+    if (saved.defined()) {
+      dq = f32(q.sizes(), k);
+      const Tensor ws = scratch(flare_causal_train_bwd_workspace_bytes(&p), k);
+      check_rc(flare_causal_train_bwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), dy.data_ptr(), saved.data_ptr(), fp(dq),
+                                      dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), st), "flare_causal_train_bwd");
+      // a batch made by expand(): autograd sums over it, so the whole gradient goes to its first entry's share
+      if (!shared && q.dim() == 3) {
+        Tensor full = at::zeros(q_.sizes(), dq.options());
+        full.select(0, 0).copy_(dq);
+        dq = full;
+      }
+    } else {
+      dq = f32({p.B, p.H, p.M, p.D}, k);
+      const Tensor ws = scratch(flare_causal_bwd_workspace_bytes(&p), k);
+      check_rc(flare_causal_bwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), dy.data_ptr(), fp(dq), dk.data_ptr(),
+                                dv.data_ptr(), fp(ws), st), "flare_causal_bwd");
+      // one latent gradient per (b, h): shared latents sum over the batch; a batch made by expand() gets the
+      // per-batch gradients, which autograd folds back itself
+      if (shared) {
+        Tensor sum = f32({p.H, p.M, p.D}, k);
+        check_rc(flare_reduce_sum(fp(dq), p.B, (int64_t)p.H * p.M, p.D, fp(sum), st), "flare_reduce_sum");
+        dq = sum;
+      }
     }
     return {as_dtype(dq, q_.scalar_type()), dk, dv, Tensor()};
   }

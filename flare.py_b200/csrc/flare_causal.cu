@@ -474,12 +474,13 @@ template <typename T, int D>
 int launch_walk(const CausalArgs& a, int n_cta_x, cudaStream_t st) {
   const size_t smem = walk_smem(a.M, D);
   if (smem > 227 * 1024) return refuse(FLARE_EUNSUPPORTED, "causal: M=%d D=%d needs %zu bytes of shared memory", a.M, D, smem);
-  cudaError_t e = cudaFuncSetAttribute(k_causal_walk<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal: %s", cudaGetErrorString(e));
+  // the limit is a property of the kernel: set to what any admitted shape may ask for, once per device
+  if (tc_set_dyn_smem(reinterpret_cast<const void*>(&k_causal_walk<T, D>), 227 * 1024) != FLARE_OK)
+    return refuse(FLARE_ECUDA, "causal: shared-memory limit could not be set");
   const dim3 grid = a.redo ? dim3((unsigned)(a.n_units < 2 * 148 ? a.n_units : 2 * 148))
                            : dim3((unsigned)n_cta_x, (unsigned)(a.B * a.H));
   launch_dep(k_causal_walk<T, D>, grid, dim3(kThreads), smem, st, a);
-  e = cudaPeekAtLastError();
+  const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal: %s", cudaGetErrorString(e));
   return FLARE_OK;
 }
@@ -531,6 +532,35 @@ int launch_causal_scan(float* rec, int n_chunks, long long rows, int D, const fl
   if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal scan: %s", cudaGetErrorString(e));
   return FLARE_OK;
 }
+
+int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc, float2* pml,
+                     const float* state_in, float* state_out, int chunks, cudaStream_t st) {
+  const int rc = causal_tc_record(p, q, k, v, pacc, pml, chunks, st);
+  if (rc != FLARE_OK) return refuse(rc, "causal: tensor-core record pass could not be launched");
+  launch_scan(true, nullptr, chunks, (long long)p->B * p->H * p->M, p->D, state_in, state_out, pacc, pml, st);
+  return FLARE_OK;
+}
+
+int causal_tc_prefill(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, __nv_bfloat16* pacc,
+                      float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st) {
+  CausalArgs a;
+  int rc = fill_args(p, &a);
+  if (rc != FLARE_OK) return rc;
+  const int chunks = (p->N + kChunk - 1) / kChunk;
+  rc = causal_tc_prefix(p, q, k, v, pacc, pml, state_in, state_out, chunks, st);
+  if (rc != FLARE_OK) return rc;
+  // the tensor-core walk flags the chunks whose scores span too many octaves for its fixed reference
+  // maximum; the fp32 walk, launched behind it, redoes exactly those (every other CTA returns at once)
+  rc = causal_tc_walk(p, q, k, v, y, pacc, pml, redo, chunks, st);
+  if (rc != FLARE_OK) return refuse(rc, "causal_prefill: tensor-core walk could not be launched");
+  const cudaError_t e = cudaPeekAtLastError();
+  if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal_prefill: %s", cudaGetErrorString(e));
+  a.q = q; a.k = k; a.v = v; a.y = y;
+  a.prefix = reinterpret_cast<const float*>(pacc);           // not read in redo mode, but marks "not a decode step"
+  a.state = nullptr; a.tokens_per_cta = kChunk;
+  a.redo = redo; a.n_units = chunks * p->B * p->H; a.pacc = pacc; a.pml = pml;
+  return run_walk(p, a, chunks, st);
+}
 }  // namespace flare
 
 extern "C" {
@@ -553,40 +583,26 @@ int flare_causal_prefill(const FlareProblem* p, const void* q, const void* k, co
   if (reinterpret_cast<uintptr_t>(workspace) % 16) return refuse(FLARE_EINVAL, "causal_prefill: workspace must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int chunks = (p->N + kChunk - 1) / kChunk;
-  // pass 1: one record per 128-token chunk
-  const bool on_tc = flare::causal_tc_walk_supported(p, q, k, v, y);
   const long long rows = (long long)p->B * p->H * p->M;
-  // workspace: fp32 records | redo flags | pml | pacc   (every piece a multiple of 16 bytes; the tensor-core path
-  // keeps its records and prefixes in the last two, the others in the first)
-  char* wsb = reinterpret_cast<char*>(workspace) + (size_t)chunks * rows * (p->D + 2) * sizeof(float);
-  int* redo = reinterpret_cast<int*>(wsb);
-  wsb += ((size_t)chunks * p->B * p->H * sizeof(int) + 15) & ~size_t(15);
-  float2* pml = reinterpret_cast<float2*>(wsb);
-  wsb += (size_t)chunks * rows * sizeof(float2);
-  __nv_bfloat16* pacc = reinterpret_cast<__nv_bfloat16*>(wsb);
-  if (on_tc) {
-    rc = flare::causal_tc_record(p, q, k, v, pacc, pml, chunks, st);
-    if (rc != FLARE_OK) return refuse(rc, "causal_prefill: tensor-core record pass could not be launched");
-  } else {
-    FlareProblem pp = *p;
-    pp.n_splits = chunks;
-    rc = flare_gather_partial(&pp, q, k, v, nullptr, workspace, st);
-    if (rc != FLARE_OK) return rc;
+  if (flare::causal_tc_walk_supported(p, q, k, v, y)) {
+    // workspace: (fp32 records of the other shapes) | redo flags | pml | pacc, every piece a multiple of 16 bytes
+    char* wsb = reinterpret_cast<char*>(workspace) + (size_t)chunks * rows * (p->D + 2) * sizeof(float);
+    int* redo = reinterpret_cast<int*>(wsb);
+    wsb += ((size_t)chunks * p->B * p->H * sizeof(int) + 15) & ~size_t(15);
+    float2* pml = reinterpret_cast<float2*>(wsb);
+    wsb += (size_t)chunks * rows * sizeof(float2);
+    return flare::causal_tc_prefill(p, q, k, v, y, reinterpret_cast<__nv_bfloat16*>(wsb), pml, redo, state_in, state_out, st);
   }
+  // pass 1: one record per 128-token chunk
+  FlareProblem pp = *p;
+  pp.n_splits = chunks;
+  rc = flare_gather_partial(&pp, q, k, v, nullptr, workspace, st);
+  if (rc != FLARE_OK) return rc;
   // pass 2: exclusive prefix along the chunk axis
-  launch_scan(true, workspace, chunks, rows, p->D, state_in, state_out, on_tc ? pacc : nullptr, on_tc ? pml : nullptr, st);
+  launch_scan(true, workspace, chunks, rows, p->D, state_in, state_out, nullptr, nullptr, st);
   // pass 3: the tokens of every chunk
   a.q = q; a.k = k; a.v = v; a.y = y;
   a.prefix = workspace; a.state = nullptr; a.tokens_per_cta = kChunk;
-  if (on_tc) {
-    // the tensor-core walk flags the chunks whose scores span too many octaves for its fixed reference
-    // maximum; the fp32 walk, launched behind it, redoes exactly those (every other CTA returns at once)
-    rc = flare::causal_tc_walk(p, q, k, v, y, pacc, pml, redo, chunks, st);
-    if (rc != FLARE_OK) return refuse(rc, "causal_prefill: tensor-core walk could not be launched");
-    const cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal_prefill: %s", cudaGetErrorString(e));
-    a.redo = redo; a.n_units = chunks * p->B * p->H; a.pacc = pacc; a.pml = pml;
-  }
   return run_walk(p, a, chunks, st);
 }
 

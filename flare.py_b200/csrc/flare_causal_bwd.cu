@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cuda_runtime.h>
 #include "common.cuh"
+#include "launch.h"
 
 namespace flare { void set_last_error(const char* msg); }
 
@@ -57,7 +58,12 @@ struct CausalBwdArgs {
   void* dk; void* dv;
   float* dq;                   // [B][H][M][D] fp32: this (b, h)'s latent gradient
   const float* prefix;         // [n_chunks][B][H][M][D+2]: the record before each chunk
-  float* sub;                  // [B*H][3][M][D+2]: records before sub-chunks 1..3 of the current chunk
+  float* sub;                  // [B*H][4][M][D+2]: records before sub-chunks 1..3 of the current chunk; slot 3 (redo): the chunk's own
+  // behind the tensor-core backward: only the (b, h) whose flag is set, their prefixes in the 16-bit form
+  const int* redo;
+  const __nv_bfloat16* pacc;   // [n_chunks][B][H][M][D]
+  const float2* pml;           // [n_chunks][B][H][M]
+  int units;                   // redo: dq holds this many partials [B*H][D/4][128][4], unscaled: this kernel's in the first, zeros in the others
 };
 
 __device__ __forceinline__ float exp_or_zero(float from, float to) {   // e^{from - to}, 0 for an empty prefix
@@ -131,13 +137,14 @@ k_causal_bwd(CausalBwdArgs a) {
 
   const int tid = threadIdx.x;
   const int bh = blockIdx.x, b = bh / a.H, h = bh % a.H;
+  if (a.redo && a.redo[bh] == 0) return;
   const T* qp = reinterpret_cast<const T*>(a.q) + b * a.qs[0] + h * a.qs[1];
   const T* kp = reinterpret_cast<const T*>(a.k) + b * a.ks[0] + h * a.ks[1];
   const T* vp = reinterpret_cast<const T*>(a.v) + b * a.vs[0] + h * a.vs[1];
   const T* gp = reinterpret_cast<const T*>(a.dy) + b * a.gs[0] + h * a.gs[1];
   T* dkp = reinterpret_cast<T*>(a.dk) + b * a.dks[0] + h * a.dks[1];
   T* dvp = reinterpret_cast<T*>(a.dv) + b * a.dvs[0] + h * a.dvs[1];
-  float* subst = a.sub + (long long)bh * 3 * M * W;
+  float* subst = a.sub + (long long)bh * 4 * M * W;
   const int MD = M * D;
 
   for (int i = tid; i < MD; i += kThreads) {
@@ -170,7 +177,15 @@ k_causal_bwd(CausalBwdArgs a) {
   for (int c = chunks - 1; c >= 0; --c) {
     const int n0 = c * kChunk, n1 = min(a.N, n0 + kChunk);
     const int nsub = (n1 - n0 + kSub - 1) / kSub;
-    const float* pre = a.prefix + (((long long)c * a.B + b) * a.H + h) * M * W;
+    const long long prow = (((long long)c * a.B + b) * a.H + h) * M;
+    const float* pre = a.prefix + prow * W;
+    if (a.redo) {
+      float* own = subst + 3LL * M * W;
+      for (int i = tid; i < MD; i += kThreads) own[(i / D) * W + i % D] = to_f32(a.pacc[prow * D + i]);
+      for (int m = tid; m < M; m += kThreads) { own[m * W + D] = a.pml[prow + m].x; own[m * W + D + 1] = a.pml[prow + m].y; }
+      pre = own;
+      __syncthreads();
+    }
 
     // ---- forward sweep: the records before sub-chunks 1 .. nsub-1 -----------------------------------
     for (int j = 0; j + 1 < nsub; ++j) {
@@ -328,16 +343,26 @@ k_causal_bwd(CausalBwdArgs a) {
       __syncthreads();
     }
   }
-  float* dq = a.dq + (long long)bh * MD;
-  {
-    const int nr = (M + 3) / 4, nc = D / 4;
-    if (tid < nr * nc) {
-      const int rt = tid / nc, ct = tid % nc;
+  const int nr = (M + 3) / 4, nc = D / 4;
+  const bool mine = tid < nr * nc;
+  const int rt = tid / nc, ct = tid % nc;
+  if (!a.redo) {
+    float* dq = a.dq + (long long)bh * MD;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        if (mine && rt + i * nr < M) dq[(rt + i * nr) * D + ct + jj * nc] = dqr[4 * i + jj] * a.scale;
+  } else {
+    for (int u = 0; u < a.units; ++u) {
+      float* dq = a.dq + ((long long)u * a.B * a.H + bh) * D * 128;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj)
-          if (rt + i * nr < M) dq[(rt + i * nr) * D + ct + jj * nc] = dqr[4 * i + jj] * a.scale;
+        for (int jj = 0; jj < 4; ++jj) {
+          const int m = rt + i * nr, d = ct + jj * nc;
+          if (mine && m < M) dq[((d >> 2) * 128 + m) * 4 + (d & 3)] = u == 0 ? dqr[4 * i + jj] : 0.f;
+        }
     }
   }
 }
@@ -349,10 +374,11 @@ size_t bwd_smem(int M, int D) {
 template <typename T, int D>
 int launch_d(const CausalBwdArgs& a, cudaStream_t st) {
   const size_t smem = bwd_smem(a.M, D);
-  cudaError_t e = cudaFuncSetAttribute(k_causal_bwd<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal_bwd: %s", cudaGetErrorString(e));
+  // the limit is a property of the kernel: set to what any admitted shape may ask for, once per device
+  if (tc_set_dyn_smem(reinterpret_cast<const void*>(&k_causal_bwd<T, D>), 227 * 1024) != FLARE_OK)
+    return refuse(FLARE_ECUDA, "causal_bwd: shared-memory limit could not be set");
   k_causal_bwd<T, D><<<(unsigned)(a.B * a.H), kThreads, smem, st>>>(a);
-  e = cudaPeekAtLastError();
+  const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal_bwd: %s", cudaGetErrorString(e));
   return FLARE_OK;
 }
@@ -367,13 +393,67 @@ int launch(const CausalBwdArgs& a, cudaStream_t st) {
   return refuse(FLARE_EUNSUPPORTED, "causal_bwd: head dim %d not in {16,32,64}", a.D);
 }
 
+CausalBwdArgs fill(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, void* dk, void* dv) {
+  CausalBwdArgs a{};
+  a.B = p->B; a.H = p->H; a.N = p->N; a.M = p->M; a.D = p->D; a.scale = p->scale;
+  for (int i = 0; i < 3; ++i) {
+    a.qs[i] = p->q_stride[i]; a.ks[i] = p->k_stride[i]; a.vs[i] = p->v_stride[i];
+    a.gs[i] = p->dy_stride[i]; a.dks[i] = p->dk_stride[i]; a.dvs[i] = p->dv_stride[i];
+  }
+  a.q = q; a.k = k; a.v = v; a.dy = dy; a.dk = dk; a.dv = dv;
+  a.units = 1;
+  return a;
+}
+
+int check_args(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const float* dq32,
+               const void* dk, const void* dv, const void* workspace) {
+  if (!p) return refuse(FLARE_EINVAL, "causal_bwd: null problem");
+  if (!q || !k || !v || !dy || !dq32 || !dk || !dv || !workspace) return refuse(FLARE_EINVAL, "causal_bwd: null pointer");
+  if (p->B < 1 || p->H < 1 || p->M < 1 || p->N < 1) return refuse(FLARE_EINVAL, "causal_bwd: bad sizes");
+  if (!(p->scale > 0.f)) return refuse(FLARE_EINVAL, "causal_bwd: scale must be > 0");
+  return FLARE_OK;
+}
+
+// The compact prefixes inside a caller's buffer: redo flags of the forward walk | (m, l) pairs | acc rows.
+struct Prefix {
+  float2* pml;
+  __nv_bfloat16* pacc;
+  int* redo;
+  Prefix(const FlareProblem* p, void* saved) {
+    const size_t chunks = ((size_t)p->N + kChunk - 1) / kChunk, BH = (size_t)p->B * p->H;
+    char* w = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(saved) + 15) & ~uintptr_t(15));
+    redo = reinterpret_cast<int*>(w);
+    w += (chunks * BH * sizeof(int) + 15) & ~size_t(15);
+    pml = reinterpret_cast<float2*>(w);
+    pacc = reinterpret_cast<__nv_bfloat16*>(w + chunks * BH * p->M * sizeof(float2));
+  }
+  static size_t bytes(const FlareProblem* p) {
+    const size_t chunks = ((size_t)p->N + kChunk - 1) / kChunk, BH = (size_t)p->B * p->H;
+    return ((chunks * BH * sizeof(int) + 15) & ~size_t(15)) + chunks * BH * p->M * (sizeof(float2) + 2 * (size_t)p->D) + 32;
+  }
+};
+
+// the shapes whose backward runs on the tensor cores, whatever the pointers
+bool tc_shape(const FlareProblem* p) {
+  return p && p->dtype == FLARE_BF16 && p->M >= 1 && p->M <= 128 && (p->D == 32 || p->D == 64) && p->N >= 1;
+}
+
 }  // namespace
 
 // pass 2 of the forward (flare_causal.cu): exclusive prefix of the chunk records, in place
 namespace flare {
 int launch_causal_scan(float* rec, int n_chunks, long long rows, int D, const float* state_in, float* state_out,
                        cudaStream_t st);
+
+int causal_bwd_redo(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
+                    const __nv_bfloat16* pacc, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
+                    void* dv, float* sub, cudaStream_t st) {
+  CausalBwdArgs a = fill(p, q, k, v, dy, dk, dv);
+  a.dq = dq_part; a.units = units; a.sub = sub;
+  a.redo = redo; a.pacc = pacc; a.pml = pml;
+  return launch<__nv_bfloat16>(a, st);
 }
+}  // namespace flare
 
 extern "C" {
 
@@ -381,15 +461,15 @@ size_t flare_causal_bwd_workspace_bytes(const FlareProblem* p) {
   if (!p || p->N < 1) return 0;
   const size_t chunks = ((size_t)p->N + kChunk - 1) / kChunk;
   const size_t rec = (size_t)p->B * p->H * p->M * (p->D + 2) * sizeof(float);
-  return chunks * rec + 3 * rec + 512;
+  const size_t simt = chunks * rec + 4 * rec + 512;
+  const size_t tc = tc_shape(p) ? Prefix::bytes(p) + causal_bwd_tc_workspace(p) + 512 : 0;
+  return simt > tc ? simt : tc;
 }
 
 int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
                      float* dq32, void* dk, void* dv, float* workspace, flare_stream_t stream) {
-  if (!p) return refuse(FLARE_EINVAL, "causal_bwd: null problem");
-  if (!q || !k || !v || !dy || !dq32 || !dk || !dv || !workspace) return refuse(FLARE_EINVAL, "causal_bwd: null pointer");
-  if (p->B < 1 || p->H < 1 || p->M < 1 || p->N < 1) return refuse(FLARE_EINVAL, "causal_bwd: bad sizes");
-  if (!(p->scale > 0.f)) return refuse(FLARE_EINVAL, "causal_bwd: scale must be > 0");
+  const int ok = check_args(p, q, k, v, dy, dq32, dk, dv, workspace);
+  if (ok != FLARE_OK) return ok;
   const int D = p->D, M = p->M;
   if (D != 16 && D != 32 && D != 64) return refuse(FLARE_EUNSUPPORTED, "causal_bwd: head dim %d not in {16,32,64}", D);
   if ((long long)M * D > (long long)kMaxDq * kThreads)
@@ -399,6 +479,15 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int chunks = (p->N + kChunk - 1) / kChunk;
   const long long rows = (long long)p->B * p->H * M;
+  if (causal_bwd_tc_supported(p, q, k, v, dy, dk, dv)) {
+    // one chunk per CTA on the tensor cores, behind the forward's record and scan passes
+    const Prefix pre(p, workspace);
+    int rc = causal_tc_prefix(p, q, k, v, pre.pacc, pre.pml, nullptr, nullptr, chunks, st);
+    if (rc == FLARE_OK)
+      rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.pml, dq32, false, dk, dv,
+                         reinterpret_cast<char*>(workspace) + Prefix::bytes(p), st);
+    return rc == FLARE_OK ? rc : refuse(rc, "causal_bwd: tensor-core pass could not be launched");
+  }
   // the forward's first two passes again: one record per 128-token chunk, then their exclusive prefix
   FlareProblem pp = *p;
   pp.n_splits = chunks;
@@ -406,13 +495,8 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
   if (rc != FLARE_OK) return rc;
   rc = launch_causal_scan(workspace, chunks, rows, D, nullptr, nullptr, st);
   if (rc != FLARE_OK) return rc;
-  CausalBwdArgs a;
-  a.B = p->B; a.H = p->H; a.N = p->N; a.M = M; a.D = D; a.scale = p->scale;
-  for (int i = 0; i < 3; ++i) {
-    a.qs[i] = p->q_stride[i]; a.ks[i] = p->k_stride[i]; a.vs[i] = p->v_stride[i];
-    a.gs[i] = p->dy_stride[i]; a.dks[i] = p->dk_stride[i]; a.dvs[i] = p->dv_stride[i];
-  }
-  a.q = q; a.k = k; a.v = v; a.dy = dy; a.dk = dk; a.dv = dv; a.dq = dq32;
+  CausalBwdArgs a = fill(p, q, k, v, dy, dk, dv);
+  a.dq = dq32;
   a.prefix = workspace;
   a.sub = workspace + (size_t)chunks * rows * (D + 2);
   switch (p->dtype) {
@@ -421,6 +505,30 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
     case FLARE_BF16: return launch<__nv_bfloat16>(a, st);
   }
   return refuse(FLARE_EINVAL, "causal_bwd: bad dtype %d", p->dtype);
+}
+
+size_t flare_causal_train_bytes(const FlareProblem* p) { return tc_shape(p) ? Prefix::bytes(p) : 0; }
+
+size_t flare_causal_train_bwd_workspace_bytes(const FlareProblem* p) { return tc_shape(p) ? causal_bwd_tc_workspace(p) : 0; }
+
+int flare_causal_train_fwd(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, void* saved,
+                           flare_stream_t stream) {
+  if (!p || !q || !k || !v || !y || !saved) return refuse(FLARE_EINVAL, "causal_train_fwd: null pointer");
+  if (!causal_tc_walk_supported(p, q, k, v, y)) return refuse(FLARE_EUNSUPPORTED, "causal_train_fwd: bf16, M <= 128, D in {32,64}, 16-byte aligned rows only");
+  const Prefix pre(p, saved);
+  return causal_tc_prefill(p, q, k, v, y, pre.pacc, pre.pml, pre.redo, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int flare_causal_train_bwd(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const void* saved,
+                           float* dq32, void* dk, void* dv, void* workspace, flare_stream_t stream) {
+  const int ok = check_args(p, q, k, v, dy, dq32, dk, dv, workspace);
+  if (ok != FLARE_OK) return ok;
+  if (!saved) return refuse(FLARE_EINVAL, "causal_train_bwd: null pointer");
+  if (!causal_bwd_tc_supported(p, q, k, v, dy, dk, dv))
+    return refuse(FLARE_EUNSUPPORTED, "causal_train_bwd: bf16, M <= 128, D in {32,64}, 16-byte aligned rows only");
+  const Prefix pre(p, const_cast<void*>(saved));
+  const int rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.pml, dq32, p->q_stride[0] == 0, dk, dv, workspace, static_cast<cudaStream_t>(stream));
+  return rc == FLARE_OK ? rc : refuse(rc, "causal_train_bwd: tensor-core pass could not be launched");
 }
 
 }  // extern "C"

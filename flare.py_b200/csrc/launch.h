@@ -82,6 +82,24 @@ int causal_tc_record(const FlareProblem* p, const void* q, const void* k, const 
 int causal_tc_walk(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, const __nv_bfloat16* pacc,
                    const float2* pml, int* redo, int chunks, cudaStream_t st);
 
+// Causal backward on the tensor cores (flare_causal_bwd_tc.cu), same shapes; pacc, pml: the prefixes the forward's scan
+// wrote.  dq32: [B][H][M][D], or [H][M][D] summed over the batch.
+bool causal_bwd_tc_supported(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
+                             const void* dk, const void* dv);
+size_t causal_bwd_tc_workspace(const FlareProblem* p);
+int causal_bwd_tc(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const __nv_bfloat16* pacc,
+                  const float2* pml, float* dq32, bool sum_batch, void* dk, void* dv, void* workspace, cudaStream_t st);
+// the fp32 backward of the (b, h) whose redo flag is set; their dq goes to partial 0 of dq_part, zeros to the others
+int causal_bwd_redo(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
+                    const __nv_bfloat16* pacc, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
+                    void* dv, float* sub, cudaStream_t st);
+// the whole prefill of the tensor-core shapes (flare_causal.cu); redo: int [chunks][B*H]
+int causal_tc_prefill(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, __nv_bfloat16* pacc,
+                      float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st);
+// record and scan passes of the prefill (flare_causal.cu): the prefix of every chunk into pacc, pml
+int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc, float2* pml,
+                     const float* state_in, float* state_out, int chunks, cudaStream_t st);
+
 // Causal linear attention on the tensor cores (flare_causal_linear_tc.cu): 16-bit inputs, Dk = 128, Dv in {32, 64}.
 bool causal_linear_tc_supported(int B, int H, int N, int Dk, int Dv, int dtype, const void* q, const int64_t* qs,
                                 const void* k, const int64_t* ks, const void* v, const int64_t* vs, const void* y,

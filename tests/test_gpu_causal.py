@@ -235,6 +235,45 @@ def test_backward_long_sequence_against_the_chunked_restatement(cuda_dev, dtype,
     assert O.rel_l2(dv.double(), dv_ref) <= tol
 
 
+@pytest.mark.parametrize("B,H,N,M,D", [
+    (1, 2, 128, 128, 64),      # one full chunk: no state handed on
+    (2, 3, 333, 128, 64),      # ragged last chunk, latents shared by the batch
+    (1, 1, 129, 64, 64),       # a last chunk of one token, fewer latents than rows
+    (1, 2, 5, 32, 32),
+    (2, 1, 1000, 96, 32),      # a latent count that is no multiple of 64
+    (1, 64, 4800, 128, 32),    # 2432 chunks: two to a unit, units taken in several rounds
+])
+def test_backward_on_tensor_cores(cuda_dev, B, H, N, M, D):
+    """bf16 with M <= 128 and D in {32, 64}: one chunk per CTA, the suffix state handed from chunk to chunk.
+    Tolerance: the results are rounded to bf16 (1.7e-3 in the 2-norm), a acc0 three times, E and Rin once each
+    (0.7e-3 apiece at this accumulation length), everything else carries a remainder term: 2.4e-3, doubled."""
+    fb = _fb()
+    (q, k, v, dy), (y, dq, dk, dv) = _bwd_case(fb, cuda_dev, B, H, N, M, D, torch.bfloat16, 1.0, seed=N + M)
+    ref = O.causal_bwd_chunked(*(t.double() for t in (q, k, v, dy)), 1.0, chunk=128)
+    for got, want in zip((dq, dk, dv), ref):
+        assert O.rel_l2(got.double(), want) <= 5e-3
+
+
+def test_backward_hands_wide_heads_to_the_fp32_kernel(cuda_dev):
+    """Scores that climb past 64 octaves inside a chunk in one of three heads: that head is redone by the fp32
+    kernel (finite, same tolerance), the others stay as they are."""
+    fb = _fb()
+    B, H, N, M, D = 1, 3, 300, 64, 32
+    q, k, v, dy = O.make_inputs(B, H, N, M, D, dtype=torch.bfloat16, seed=29)
+    k = k.clone()
+    k[:, 1, 128:256] = (k[:, 1, 128:256].float() * torch.linspace(0.1, 40.0, 128).view(1, 128, 1)).bfloat16()
+    qd, kd, vd = (t.to(cuda_dev).requires_grad_(True) for t in (q, k, v))
+    y = fb.flare_causal_mixer(qd, kd, vd, 1.0)
+    y.backward(dy.to(cuda_dev))
+    assert fb.device_status() == 0
+    ref = O.causal_bwd_chunked(*(t.double() for t in (q, k, v, dy)), 1.0, chunk=32)
+    for got, want in zip((qd.grad, kd.grad, vd.grad), ref):
+        assert torch.isfinite(got).all()
+        for h in range(H):
+            g, r = (got[h], want[h]) if got.dim() == 3 else (got[:, h], want[:, h])
+            assert O.rel_l2(g.double().cpu(), r) <= 5e-3, h
+
+
 def test_backward_with_growing_logits(cuda_dev):
     """Keys whose norm grows along the sequence: the running maxima rise by tens of units from chunk to
     chunk, so the carried suffix state is rescaled by tiny factors and early tokens' weights underflow
