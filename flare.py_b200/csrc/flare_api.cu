@@ -48,17 +48,54 @@ int check_tok(const char* name, const void* ptr, const int64_t* st, int dtype) {
   return FLARE_OK;
 }
 
+// Estimated device time (microseconds) of the passes that run one CTA per (b, h, latent block, token range), for S ranges
+// of `tiles` 128-token tiles.  What decides is how full the last wave of CTAs is: 19 ranges for 8 heads are 152
+// one-per-SM CTAs of the backward, two waves where 18 ranges take one (1.86 -> 1.16 ms at N = 300 007, M = 512, D = 32).
+// Measured times per CTA and tile: latent-major passes 1.7 with two CTAs on the SM, 1.12 alone; one-exponential backward
+// 1.5, general backward 5.5 (per 128 latents); set-up 4 and 12 per CTA.
+double split_cost(const FlareProblem* p, bool tc, long long tiles, long long S) {
+  const long long bh = (long long)p->B * p->H, nb = (p->M + 127) / 128, per = (tiles + S - 1) / S;
+  const double parts = (double)S * bh * p->M * (p->D + 2) * 4 * 3 / 2.5e6;          // partial records written and read again
+  if (!tc) {                                                                        // fp32 kernels: about two blocks per SM
+    const long long lpb = p->D == 16 ? 64 : 128;
+    const long long grid = bh * ((p->M + lpb - 1) / lpb) * S;
+    return (double)((grid + 295) / 296) * (per + 0.3) * 4 + parts;
+  }
+  const long long grid = bh * nb * S, full = grid / 296, rem = grid % 296;
+  double lat = full * (per * 1.7 + 4);
+  if (rem) lat += per * (rem <= 148 ? 1.12 : 1.7) + 4;
+  const bool fast = p->dtype == FLARE_BF16 && p->D == 32;
+  const long long waves = (bh * S + 147) / 148, launches = (nb + 1) / 2;
+  return 2 * lat + waves * (per * nb * (fast ? 1.5 : 5.5) + 12 * launches) + parts;
+}
+
 int auto_splits(const FlareProblem* p) {
-  const int tpt = p->D <= 32 ? 1 : p->D / 32;
-  const int lpb = 128 / tpt;
-  const long long base = (long long)p->B * p->H * ((p->M + lpb - 1) / lpb);
-  long long s = (4LL * 148 + base - 1) / base;
   const long long max_s = (p->N + 127) / 128;
-  // short ranges (a context-parallel shard, a small N): one wave of CTAs instead of two, so that the
-  // per-CTA set-up (resident operands, first tiles) is paid once
-  if (max_s / s < 64) s = (2LL * 148) / base > 0 ? (2LL * 148) / base : 1;
-  if (s > max_s) s = max_s;
-  if (s > 1024) s = 1024;
+  long long s = 1;
+  if (p->D <= 32) {
+    // candidates: the largest S that fills one to four waves of one or two CTAs per SM
+    const bool tc = p->dtype != FLARE_F32 && p->D >= 16;
+    const long long bh = (long long)p->B * p->H, nb = (p->M + 127) / 128, top = max_s < 1024 ? max_s : 1024;
+    double best = 1e300;
+    for (int w = 1; w <= 4; ++w)
+      for (int i = 0; i < 3; ++i) {
+        long long cand = 148LL * w * (i > 0 ? 2 : 1) / (i < 2 ? bh : bh * nb);
+        if (i == 2 && nb == 1) continue;
+        cand = cand < 1 ? 1 : cand > top ? top : cand;
+        if (cand < 1) continue;                        // N = 0
+        const double t = split_cost(p, tc, max_s, cand);
+        if (t < best) { best = t; s = cand; }
+      }
+  } else {
+    const int lpb = 128 / (p->D / 32);
+    const long long base = (long long)p->B * p->H * ((p->M + lpb - 1) / lpb);
+    s = (4LL * 148 + base - 1) / base;
+    // short ranges (a context-parallel shard, a small N): one wave of CTAs instead of two, so that the
+    // per-CTA set-up (resident operands, first tiles) is paid once
+    if (max_s / s < 64) s = (2LL * 148) / base > 0 ? (2LL * 148) / base : 1;
+    if (s > max_s) s = max_s;
+    if (s > 1024) s = 1024;
+  }
   if (s < 1) s = 1;
   // ranges are whole multiples of 128 tokens: drop ranges that would be empty
   const long long chunk = (((p->N + s - 1) / s + 127) / 128) * 128;
