@@ -5,15 +5,20 @@
 //   dS   = P (dZ V^T - Delta_m) + A (Z dY^T - delta_n)      delta_n = dY_n . Y_n,  Delta_m = dZ_m . Z_m
 //   dV_n = sum_m P_mn dZ_m     dK_n = scale sum_m dS_mn q_m     dQ_m = scale sum_n dS_mn k_n
 //
-// One CTA (256 threads, one per SM: it uses all 512 tensor-memory columns) owns one (b, h) and
-// one token range and walks it in 128-token tiles; the latents are taken in blocks of 128.
-// Per (tile, latent block j), token-major (tensor-memory lane = token):
-//   MMA  : S^T = K_t Q_j^T,  T1 = V_t dZ_j^T,  T2 = dY_t Z_j^T      -> columns [0,128) [128,256) [256,384)
-//   SIMT : two exponentials per score; P and dS are packed to bf16 over S and T1 (each half of the
-//          threads keeps to its own 64 columns); dS also goes to shared memory, token-major rows,
-//          which is the MN-major A operand of the dQ product
-//   MMA  : dV += P^T dZ_j,  dK += dS^T Q_j   (A from tensor memory)     -> columns [384,384+D) [416,416+D)
-//          dQ_j += dS K_t                     (A and B from shared memory) -> columns [448+32j, +D)
+// One CTA owns one (b, h) and one token range and walks it in 128-token tiles; a step is one tile x SUB latents, four
+// (SUB = 128) or two (SUB = 64) threads per token row, 32 latents each.  Per step (tensor-memory lane = token):
+//   MMA  : S^T = K_t Q_s^T,  T1 = V_t dZ_s^T,  T2 = dY_t Z_s^T          -> columns [0,SUB) [SUB,2SUB) [2SUB,3SUB)
+//   SIMT : two exponentials per score; P and dS are packed to 16 bits over the thread's own columns of S and T1; dS
+//          also goes to shared memory, token-major rows, which is the MN-major A operand of the dQ product
+//   MMA  : dV += P^T dZ_s,  dK += dS^T Q_s   (A from tensor memory)      -> columns 3SUB, 3SUB + D
+//          dQ_j += dS K_t  once per 128 latents (A, B from shared memory) -> columns 3SUB + 2D + Dj
+// The products of the next step are issued right behind those of this one (products of one thread execute in issue
+// order), so a step costs one round trip through the tensor core.  What bounds the kernel is that serial chain
+// -- round trip, tensor-memory reads, exponentials, hand-over -- rather than a pipe, so for D = 16 a step is 64 latents:
+// 256 tensor-memory columns and 91 KB, and two CTAs share an SM, one's chain under the other's.  D = 32 needs all
+// 512 columns (its accumulators alone take 128) and runs one CTA of 512 threads.  With 128-latent steps, 256
+// threads, one CTA per SM and two round trips a step D = 16 took 350 us instead of 172 (B = 32, H = 8, N = 4096, M = 128,
+// fp16, masked) and 81 instead of 29 (B = 4, H = 8, N = 7225, M = 64, bf16).
 // Q, Z, dZ stay resident in shared memory for the whole range, each tile in one layout that
 // serves both as a K-major and as an MN-major operand.  K, V, dY, Y tiles arrive by TMA in a
 // two-stage ring.
@@ -53,6 +58,13 @@ struct BwdArgs {
   const int* flag;             // [B*H] or null: run only the (b, h) whose flag is 1
 };
 
+template <int D> struct BwdShape {
+  static constexpr int SUB = D == 16 ? 64 : 128;   // latents per step
+  static constexpr int kThreads = 4 * SUB;         // 32 score columns per thread
+  static constexpr int kCtas = D == 16 ? 2 : 1;    // per SM
+  static constexpr int kCols = D == 16 ? 256 : 512;
+};
+
 template <int D>
 struct BwdSmem {
   static constexpr int ROWB = 2 * D;
@@ -60,17 +72,19 @@ struct BwdSmem {
   static constexpr int kT = 128 * ROWB;            // one token tile
   static constexpr int kStage = 4 * kT;            // K, V, dY, Y
   static constexpr int kDS = 2 * 128 * 128;        // dS^T [2 blocks of 64 latents][128 tok][128 B]
-  static constexpr int kBytes = 3 * kLat + 2 * kStage + kDS + 256 * 8 + 2 * 128 * 8 + 2 * 128 * 4 + 1024 + 128;
+  static constexpr int kBytes = 3 * kLat + 2 * kStage + kDS + 256 * 8 + 1024 + 128;
 };
 
-template <int D, typename T16, bool ACC>          // ACC: add to the dK/dV an earlier latent block wrote
-__global__ void __launch_bounds__(256, 1)
+// ACC: add to the dK/dV an earlier latent block wrote.  PLAIN: both terms, no dropout (decided at compile time).
+template <int D, typename T16, bool ACC, bool PLAIN>
+__global__ void __launch_bounds__(BwdShape<D>::kThreads, BwdShape<D>::kCtas)
 k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG,
          const __grid_constant__ CUtensorMap tmY, BwdArgs a) {
   grid_dep_sync();
   constexpr int ROWB = 2 * D;
   constexpr int CPR = ROWB / 16;
+  constexpr int SUB = BwdShape<D>::SUB, NT = BwdShape<D>::kThreads;
   using L = BwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -80,9 +94,7 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
   uint8_t* sTok = sDZ + L::kLat;                   // [2 stages][K | V | dY | Y]
   uint8_t* sDS = sTok + 2 * L::kStage;
   float2* sLD = reinterpret_cast<float2*>(sDS + L::kDS);     // [256] {L_m log2e, Delta_m}
-  float2* sCD = sLD + 256;                                    // [2][128] {C_n log2e, delta_n}
-  float* sBias = reinterpret_cast<float*>(sCD + 256);         // [2][128] 0, or -inf for an excluded token
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + 256);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sLD + 256);
   uint64_t* bar_full = bars;                       // [2]
   uint64_t* bar_mma = bars + 2;
   uint64_t* bar_q = bars + 3;
@@ -90,21 +102,22 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
   int* abort_flag = reinterpret_cast<int*>(bars + 5);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wg = warp >> 2;                        // which 64 of the 128 columns this thread handles
+  const int cg = warp >> 2;                        // which 32 of the step's latents this thread handles
   const int row = (warp & 3) * 32 + lane;          // token within the tile = tensor-memory lane
   const int split = blockIdx.x % a.n_splits;
   const int bh = blockIdx.x / a.n_splits;
   if (a.flag && a.flag[bh] != 1) return;           // the one-exponential kernel owns this (b, h)
   const int b = bh / a.H, h = bh % a.H;
   const int M = a.M;
-  const bool use_g = (a.terms & FLARE_TERM_GATHER) != 0, use_s = (a.terms & FLARE_TERM_SCATTER) != 0;
-  const int n_mblk = (M + 127) / 128;
+  const bool use_g = PLAIN || (a.terms & FLARE_TERM_GATHER) != 0, use_s = PLAIN || (a.terms & FLARE_TERM_SCATTER) != 0;
+  const bool drop = !PLAIN && a.drop.on;
+  const int n_sub = (M + SUB - 1) / SUB, n_mblk = (M + 127) / 128;
   const int n0 = split * a.chunk, n1 = min(a.N, n0 + a.chunk);
   const int n_tiles = n1 > n0 ? (n1 - n0 + 127) / 128 : 0;
   float* dq_out = a.dq_part + ((((long long)split * a.B + b) * a.H + h) * a.M_total + a.m0) * D;
 
   if (n_tiles == 0) {                              // empty range contributes nothing
-    for (int i = tid; i < M * D; i += 256) dq_out[i] = 0.f;
+    for (int i = tid; i < M * D; i += NT) dq_out[i] = 0.f;
     return;
   }
 
@@ -115,15 +128,16 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
     fence_barrier_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmG); prefetch_tmap(&tmY);
   }
-  if (warp == 0) tmem_alloc<512>(tmem_slot);
+  if (warp == 0) tmem_alloc<BwdShape<D>::kCols>(tmem_slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t cS = 0, cT1 = 128, cT2 = 256, cDV = 384, cDK = 416, cDQ = 448;
+  constexpr uint32_t cS = 0, cT1 = SUB, cT2 = 2 * SUB, cDV = 3 * SUB, cDK = cDV + D, cDQ = cDK + D;
 
-  auto load_tile = [&](int stage, int tok0) {
+  auto load_tile = [&](int t) {
+    const int stage = t & 1, tok0 = n0 + t * 128;
     uint8_t* dst = sTok + stage * L::kStage;
     mbar_expect_tx(&bar_full[stage], (1 + (use_g ? 1 : 0) + (use_s ? 2 : 0)) * L::kT);
     tma_load_4d(dst, &tmK, &bar_full[stage], 0, tok0, h, b);
@@ -137,16 +151,17 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
   if (tid == 0) {
     mbar_expect_tx(bar_q, L::kLat);
     tma_load_4d(sQ, &tmQ, bar_q, 0, 0, h, a.q_batched ? b : 0);       // rows past M arrive as zeros
-    load_tile(0, n0);
+    load_tile(0);
+    if (n_tiles > 1) load_tile(1);
   }
-  // resident latent operands: Z and dZ as bf16 in the swizzled tile layout; L and Delta per latent
+  // resident latent operands: Z and dZ as 16-bit in the swizzled tile layout; L and Delta per latent
   {
     const long long lrow = ((long long)b * a.H + h) * a.M_total + a.m0;
     const float* zb = a.z32 + lrow * D;
     const float* dzb = use_g ? a.dz32 + lrow * D : nullptr;
     // CPR consecutive lanes share a latent row (eight values each): coalesced reads, and Delta_m = dZ_m . Z_m is
     // summed over them by shuffles (whole warps run every iteration)
-    for (int i = tid; i < 256 * CPR; i += 256) {
+    for (int i = tid; i < 256 * CPR; i += NT) {
       const int r = i / CPR, c = i % CPR;
       uint4 pz = make_uint4(0, 0, 0, 0), pd = make_uint4(0, 0, 0, 0);
       float dl = 0.f;
@@ -182,10 +197,9 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
   }
   fence_proxy_async();
   __syncthreads();
-  mbar_wait(bar_q, 0, a.status, abort_flag);
 
   constexpr int F = Op16<T16>::kFmt;
-  const uint32_t id_st = idesc_f16(128, 128, F, F, 0, 0);    // S^T, T1, T2: A, B K-major
+  const uint32_t id_st = idesc_f16(128, SUB, F, F, 0, 0);    // S^T, T1, T2: A, B K-major
   const uint32_t id_tv = idesc_f16(128, D, F, F, 0, 1);      // dV, dK: A in tensor memory, B MN-major
   const uint32_t id_dq = idesc_f16(128, D, F, F, 1, 1);      // dQ: A and B MN-major
   const float sl = a.scale_log2;
@@ -194,77 +208,148 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
   uint32_t ph_mma = 0;
   bool aborted = false;
 
+  // S^T, T1, T2 of step (t, s); warp 0, whole warp converged around the elected lane
+  auto issue_scores = [&](int t, int s) {
+    const uint8_t* tK = sTok + (t & 1) * L::kStage;
+    const uint64_t dK_ = smem_desc<ROWB>(smem_u32(tK)), dV_ = smem_desc<ROWB>(smem_u32(tK + L::kT)),
+                   dG_ = smem_desc<ROWB>(smem_u32(tK + 2 * L::kT));
+    const uint32_t lo = (uint32_t)(s * SUB * ROWB);
+    const uint64_t dQ_ = smem_desc<ROWB>(smem_u32(sQ) + lo), dZ_ = smem_desc<ROWB>(smem_u32(sZ) + lo),
+                   dDZ_ = smem_desc<ROWB>(smem_u32(sDZ) + lo);
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cS, dK_ + 2 * kk, dQ_ + 2 * kk, id_st, kk > 0);
+    if (use_g) {
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cT1, dV_ + 2 * kk, dDZ_ + 2 * kk, id_st, kk > 0);
+    }
+    if (use_s) {
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cT2, dG_ + 2 * kk, dZ_ + 2 * kk, id_st, kk > 0);
+    }
+  };
+  // dV, dK of step (t, s), and dQ of a 128-latent block whose dS is complete
+  auto issue_grads = [&](int t, int s) {
+    const uint32_t lo = (uint32_t)(s * SUB * ROWB);
+    const uint64_t bDZ = smem_desc<ROWB>(smem_u32(sDZ) + lo), bQ = smem_desc<ROWB>(smem_u32(sQ) + lo);
+#pragma unroll
+    for (int kk = 0; kk < SUB / 16; ++kk) {        // contraction over the latents of the step
+      const uint32_t acol = 32 * (kk >> 1) + 8 * (kk & 1);
+      const uint64_t boff = (uint64_t)((kk * 16 * ROWB) >> 4);
+      if (use_g) mma_ts(tmem + cDV, tmem + cS + acol, bDZ + boff, id_tv, (s > 0) || (kk > 0));
+      mma_ts(tmem + cDK, tmem + cT1 + acol, bQ + boff, id_tv, (s > 0) || (kk > 0));
+    }
+    // (latents past M of a half-filled block: rows of dQ that are never stored)
+    if (SUB == 128 || (s & 1) || s == n_sub - 1) {
+      const uint64_t bK = smem_desc<ROWB>(smem_u32(sTok + (t & 1) * L::kStage));
+      const uint64_t aDS = smem_desc_mn128(smem_u32(sDS), 128 * 128, 1024);
+      const uint32_t d = tmem + cDQ + D * (s * SUB / 128);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)               // contraction over the 128 tokens of the tile
+        mma_ss(d, aDS + (uint64_t)((kk * 2048) >> 4), bK + (uint64_t)((kk * 16 * ROWB) >> 4), id_dq, (t > 0) || (kk > 0));
+    }
+  };
+  // dV (column group 0) and dK (group 1) of finished tile t -> global
+  auto store_tile = [&](int t) {
+    if (cg > 1 || (cg == 0 && !use_g)) return;
+    uint32_t r[D];
+    const uint32_t col = cg ? cDK : cDV;
+    if constexpr (D == 16) tmem_ld16(lane_base + col, r);
+    else tmem_ld32(lane_base + col, r);
+    tmem_wait_ld();
+    const int n = n0 + t * 128 + row;
+    if (n < n1) {
+      const float f = cg ? a.scale : 1.f;
+      uint16_t* op = cg ? static_cast<uint16_t*>(a.dk) + b * a.dks[0] + h * a.dks[1] + (long long)n * a.dks[2]
+                        : static_cast<uint16_t*>(a.dv) + b * a.dvs[0] + h * a.dvs[1] + (long long)n * a.dvs[2];
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c) {
+        float g[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] = __uint_as_float(r[8 * c + j]) * f;
+        if constexpr (ACC) {
+          const uint4 old = reinterpret_cast<const uint4*>(op)[c];
+          const uint32_t* o2 = reinterpret_cast<const uint32_t*>(&old);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 of = Op16<T16>::unpack(o2[j]);
+            g[2 * j] += of.x; g[2 * j + 1] += of.y;
+          }
+        }
+        uint4 o;
+        o.x = Op16<T16>::pack(g[0], g[1]); o.y = Op16<T16>::pack(g[2], g[3]);
+        o.z = Op16<T16>::pack(g[4], g[5]); o.w = Op16<T16>::pack(g[6], g[7]);
+        reinterpret_cast<uint4*>(op)[c] = o;
+      }
+    }
+  };
+
+  mbar_wait(bar_q, 0, a.status, abort_flag);
+  if (warp == 0) {
+    mbar_wait(&bar_full[0], 0, a.status, abort_flag);
+    tc_fence_after();
+    if (elect_one()) { issue_scores(0, 0); mma_commit(bar_mma); }
+    __syncwarp();
+  }
+
+  // keep flag and C_n of this thread's token, fetched a tile ahead
+  bool keep_next;
+  float c_next;
+  auto fetch_token = [&](int t) {
+    const int n = n0 + t * 128 + row;
+    keep_next = n < n1 && (!mrow || mrow[n] != 0);
+    c_next = keep_next && use_s ? cb[n] : 0.f;
+  };
+  fetch_token(0);
+
   for (int t = 0; t < n_tiles && !aborted; ++t) {
-    const int st = t & 1;
-    const int tok0 = n0 + t * 128;
-    uint8_t* tK = sTok + st * L::kStage;
-    uint8_t* tV = tK + L::kT;
-    uint8_t* tG = tK + 2 * L::kT;
-    uint8_t* tY = tK + 3 * L::kT;
-    if (tid == 0 && t + 1 < n_tiles) load_tile(st ^ 1, tok0 + 128);   // every MMA of tile t-1 is complete
+    const int st = t & 1, n = n0 + t * 128 + row;
+    const uint8_t* tG = sTok + st * L::kStage + 2 * L::kT;
+    const uint8_t* tY = tG + L::kT;
     mbar_wait(&bar_full[st], (uint32_t)(t >> 1) & 1, a.status, abort_flag);
 
     // per-token scalars: C_n (log2 units) and delta_n = dY_n . Y_n from the tiles just loaded; the score
     // bias that removes a token (past the end of the range, or masked out): P = A = 0 for it
-    if (tid < 128) {
-      const int n = tok0 + tid;
-      float dl = 0.f, c2 = INFINITY;
-      const bool keep = n < n1 && (!mrow || mrow[n] != 0);
-      if (keep && use_s) {
+    const bool keep = keep_next;
+    const float c_tok = c_next;
+    fetch_token(t + 1);
+    const float bias = keep ? 0.f : -INFINITY;
+    float deln = 0.f, c2n = INFINITY;
+    if (keep && use_s) {
+      c2n = c_tok * kLog2e;
 #pragma unroll
-        for (int c = 0; c < CPR; ++c) {
-          const uint4 g4 = *reinterpret_cast<const uint4*>(tG + swz_off<ROWB>(tid, c));
-          const uint4 y4 = *reinterpret_cast<const uint4*>(tY + swz_off<ROWB>(tid, c));
-          const uint32_t* gp = reinterpret_cast<const uint32_t*>(&g4);
-          const uint32_t* yp = reinterpret_cast<const uint32_t*>(&y4);
+      for (int c = 0; c < CPR; ++c) {
+        const uint4 g4 = *reinterpret_cast<const uint4*>(tG + swz_off<ROWB>(row, c));
+        const uint4 y4 = *reinterpret_cast<const uint4*>(tY + swz_off<ROWB>(row, c));
+        const uint32_t* gp = reinterpret_cast<const uint32_t*>(&g4);
+        const uint32_t* yp = reinterpret_cast<const uint32_t*>(&y4);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 gf = Op16<T16>::unpack(gp[j]), yf = Op16<T16>::unpack(yp[j]);
-            dl = fmaf(gf.x, yf.x, dl); dl = fmaf(gf.y, yf.y, dl);
-          }
+        for (int j = 0; j < 4; ++j) {
+          const float2 gf = Op16<T16>::unpack(gp[j]), yf = Op16<T16>::unpack(yp[j]);
+          deln = fmaf(gf.x, yf.x, deln); deln = fmaf(gf.y, yf.y, deln);
         }
-        c2 = cb[n] * kLog2e;
       }
-      sCD[st * 128 + tid] = make_float2(c2, dl);
-      sBias[st * 128 + tid] = keep ? 0.f : -INFINITY;
     }
-    __syncthreads();
-    const float2 cd = sCD[st * 128 + row];
-    const float c2n = cd.x, deln = cd.y, bias = sBias[st * 128 + row];
-    const uint32_t ntok = (uint32_t)(tok0 + row);
+    const uint32_t ntok = (uint32_t)n;
     const uint32_t drow_g = (uint32_t)(1 * a.B * a.H + bh) * (uint32_t)a.M_total;     // gather weights' rows
     const uint32_t drow_s = (uint32_t)(2 * a.B * a.H + bh) * (uint32_t)a.M_total;     // scatter weights' rows
 
-    for (int j = 0; j < n_mblk; ++j) {
-      if (tid == 0) {
-        tc_fence_after();
-        const uint64_t dK_ = smem_desc<ROWB>(smem_u32(tK)), dV_ = smem_desc<ROWB>(smem_u32(tV)),
-                       dG_ = smem_desc<ROWB>(smem_u32(tG));
-        const uint32_t lo = (uint32_t)(j * 128 * ROWB);
-        const uint64_t dQ_ = smem_desc<ROWB>(smem_u32(sQ) + lo), dZ_ = smem_desc<ROWB>(smem_u32(sZ) + lo),
-                       dDZ_ = smem_desc<ROWB>(smem_u32(sDZ) + lo);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cS, dK_ + 2 * kk, dQ_ + 2 * kk, id_st, kk > 0);
-        if (use_g) {
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cT1, dV_ + 2 * kk, dDZ_ + 2 * kk, id_st, kk > 0);
-        }
-        if (use_s) {
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cT2, dG_ + 2 * kk, dZ_ + 2 * kk, id_st, kk > 0);
-        }
-        mma_commit(bar_mma);
-      }
-      mbar_wait(bar_mma, ph_mma, a.status, abort_flag);
+    for (int s = 0; s < n_sub; ++s) {
+      // the scores of this step are there, and with them every product issued earlier is complete
+      mbar_wait_hot(bar_mma, ph_mma, a.status, abort_flag);
       ph_mma ^= 1;
       tc_fence_after();
+      if (s == 0 && t > 0) {
+        if (tid == 0 && t + 1 < n_tiles) load_tile(t + 1);   // into the stage of tile t-1
+        store_tile(t - 1);
+      }
 
-      // ---- P, A, dS for this thread's token and its 64 latents of block j ---------------------
-      const uint32_t colb = 64 * wg;
-      const float2* ld = sLD + j * 128 + colb;
-      uint8_t* ds_row = sDS + wg * (128 * 128);    // MN block wg: [128 tok][128 B]
+      // ---- P, A, dS for this thread's token and its 32 latents of the step ---------------------
+      const uint32_t colb = 32 * cg;
+      const float2* ld = sLD + s * SUB + colb;
+      const int l128 = (s * SUB + (int)colb) & 127;
+      uint8_t* ds_row = sDS + (l128 >> 6) * (128 * 128);    // MN block: [128 tok][128 B]
 #pragma unroll 1
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
         uint32_t rs[16], r1[16], r2[16], pp[8], pd[8];
         tmem_ld16(lane_base + cS + colb + 16 * i, rs);
         if (use_g) tmem_ld16(lane_base + cT1 + colb + 16 * i, r1);
@@ -273,38 +358,38 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const float4 l4 = *reinterpret_cast<const float4*>(&ld[16 * i + 2 * e]);   // {L2,Dl} x 2
-          const float x0 = fmaf(__uint_as_float(rs[2 * e]), sl, bias), x1 = fmaf(__uint_as_float(rs[2 * e + 1]), sl, bias);
-          float p0 = ex2(x0 - l4.x), p1 = ex2(x1 - l4.z);
-          float t10 = __uint_as_float(r1[2 * e]), t11 = __uint_as_float(r1[2 * e + 1]);
-          float t20 = __uint_as_float(r2[2 * e]), t21 = __uint_as_float(r2[2 * e + 1]);
-          float pv0 = p0, pv1 = p1;                 // the weights dV sees
-          if (a.drop.on) {
+          const float2 x = __ffma2_rn(make_float2(__uint_as_float(rs[2 * e]), __uint_as_float(rs[2 * e + 1])),
+                                      make_float2(sl, sl), make_float2(bias, bias));
+          const float2 xp = __fadd2_rn(x, make_float2(-l4.x, -l4.z));
+          float2 pv = make_float2(ex2(xp.x), ex2(xp.y));             // the weights dV sees
+          const float2 p = pv;
+          float2 t1 = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+          float2 t2 = make_float2(__uint_as_float(r2[2 * e]), __uint_as_float(r2[2 * e + 1]));
+          if (drop) {
             // z = (D1 P / (1-p)) V and y = (D2 A / (1-p))^T z: the upstream factors dZ V^T and Z dY^T pass the
             // same masks before Delta_m = dZ_m . Z_m and delta_n = dY_n . Y_n are subtracted
-            const uint32_t mcol = (uint32_t)(a.m0 + j * 128 + colb + 16 * i + 2 * e);
+            const uint32_t mcol = (uint32_t)(a.m0 + s * SUB + colb + 16 * i + 2 * e);
             const float k10 = drop_hash(ntok, drow_g + mcol, a.drop.seed_lo, a.drop.seed_hi) >= a.drop.thresh ? a.drop.inv_keep : 0.f;
             const float k11 = drop_hash(ntok, drow_g + mcol + 1, a.drop.seed_lo, a.drop.seed_hi) >= a.drop.thresh ? a.drop.inv_keep : 0.f;
             const float k20 = drop_hash(ntok, drow_s + mcol, a.drop.seed_lo, a.drop.seed_hi) >= a.drop.thresh ? a.drop.inv_keep : 0.f;
             const float k21 = drop_hash(ntok, drow_s + mcol + 1, a.drop.seed_lo, a.drop.seed_hi) >= a.drop.thresh ? a.drop.inv_keep : 0.f;
-            pv0 *= k10; pv1 *= k11; t10 *= k10; t11 *= k11; t20 *= k20; t21 *= k21;
+            pv.x *= k10; pv.y *= k11; t1.x *= k10; t1.y *= k11; t2.x *= k20; t2.y *= k21;
           }
-          float s0 = 0.f, s1 = 0.f;
+          float2 ds = make_float2(0.f, 0.f);
           if (use_s) {
-            const float a0 = ex2(x0 - c2n), a1 = ex2(x1 - c2n);
-            s0 = a0 * (t20 - deln);
-            s1 = a1 * (t21 - deln);
+            const float2 xa = __fadd2_rn(x, make_float2(-c2n, -c2n));
+            const float2 d2 = __fadd2_rn(t2, make_float2(-deln, -deln));
+            ds = __fmul2_rn(make_float2(ex2(xa.x), ex2(xa.y)), d2);
           }
-          if (use_g) {
-            s0 = fmaf(p0, t10 - l4.y, s0);
-            s1 = fmaf(p1, t11 - l4.w, s1);
-          }
-          pp[e] = Op16<T16>::pack(pv0, pv1);
-          pd[e] = Op16<T16>::pack(s0, s1);
+          if (use_g) ds = __ffma2_rn(p, __fadd2_rn(t1, make_float2(-l4.y, -l4.w)), ds);
+          pp[e] = Op16<T16>::pack(pv.x, pv.y);
+          pd[e] = Op16<T16>::pack(ds.x, ds.y);
         }
         tmem_st8(lane_base + cS + colb + 8 * i, pp);
         tmem_st8(lane_base + cT1 + colb + 8 * i, pd);
-        *reinterpret_cast<uint4*>(ds_row + swz_off<128>(row, 2 * i)) = make_uint4(pd[0], pd[1], pd[2], pd[3]);
-        *reinterpret_cast<uint4*>(ds_row + swz_off<128>(row, 2 * i + 1)) = make_uint4(pd[4], pd[5], pd[6], pd[7]);
+        const int ch = ((l128 & 63) >> 3) + 2 * i;
+        *reinterpret_cast<uint4*>(ds_row + swz_off<128>(row, ch)) = make_uint4(pd[0], pd[1], pd[2], pd[3]);
+        *reinterpret_cast<uint4*>(ds_row + swz_off<128>(row, ch + 1)) = make_uint4(pd[4], pd[5], pd[6], pd[7]);
       }
       tmem_wait_st();
       fence_proxy_async();
@@ -313,86 +398,43 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
       aborted = *reinterpret_cast<volatile int*>(abort_flag) != 0;
       if (aborted) break;
 
-      if (tid == 0) {
+      if (warp == 0) {
+        const bool last = s == n_sub - 1, more = !last || t + 1 < n_tiles;
+        if (last && more) mbar_wait_hot(&bar_full[st ^ 1], (uint32_t)((t + 1) >> 1) & 1, a.status, abort_flag);
         tc_fence_after();
-        const uint32_t lo = (uint32_t)(j * 128 * ROWB);
-        const uint64_t bDZ = smem_desc<ROWB>(smem_u32(sDZ) + lo), bQ = smem_desc<ROWB>(smem_u32(sQ) + lo);
-        const uint64_t bK = smem_desc<ROWB>(smem_u32(tK));
-        const uint64_t aDS = smem_desc_mn128(smem_u32(sDS), 128 * 128, 1024);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {           // contraction over the 128 latents of block j
-          const uint32_t acol = (kk < 4) ? 8 * kk : 64 + 8 * (kk - 4);
-          const uint64_t boff = (uint64_t)((kk * 16 * ROWB) >> 4);
-          if (use_g) mma_ts(tmem + cDV, tmem + cS + acol, bDZ + boff, id_tv, (j > 0) || (kk > 0));
-          mma_ts(tmem + cDK, tmem + cT1 + acol, bQ + boff, id_tv, (j > 0) || (kk > 0));
+        if (elect_one()) {
+          issue_grads(t, s);
+          if (more) issue_scores(last ? t + 1 : t, last ? 0 : s + 1);
+          mma_commit(bar_mma);
         }
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)             // contraction over the 128 tokens of the tile
-          mma_ss(tmem + cDQ + 32 * j, aDS + (uint64_t)((kk * 2048) >> 4), bK + (uint64_t)((kk * 16 * ROWB) >> 4),
-                 id_dq, (t > 0) || (kk > 0));
-        mma_commit(bar_mma);
-      }
-      mbar_wait(bar_mma, ph_mma, a.status, abort_flag);
-      ph_mma ^= 1;
-      tc_fence_after();
-    }
-    if (aborted) break;
-
-    // ---- dV (first half of the threads) and dK (second half) of this tile -> global -------------
-    if (wg == 1 || use_g) {
-      uint32_t r[D];
-      const uint32_t col = wg ? cDK : cDV;
-      if constexpr (D == 16) tmem_ld16(lane_base + col, r);
-      else tmem_ld32(lane_base + col, r);
-      tmem_wait_ld();
-      const int n = tok0 + row;
-      if (n < n1) {
-        const float f = wg ? a.scale : 1.f;
-        uint16_t* op = wg ? static_cast<uint16_t*>(a.dk) + b * a.dks[0] + h * a.dks[1] + (long long)n * a.dks[2]
-                          : static_cast<uint16_t*>(a.dv) + b * a.dvs[0] + h * a.dvs[1] + (long long)n * a.dvs[2];
-#pragma unroll
-        for (int c = 0; c < D / 8; ++c) {
-          float g[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) g[j] = __uint_as_float(r[8 * c + j]) * f;
-          if constexpr (ACC) {
-            const uint4 old = reinterpret_cast<const uint4*>(op)[c];
-            const uint32_t* o2 = reinterpret_cast<const uint32_t*>(&old);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 of = Op16<T16>::unpack(o2[j]);
-              g[2 * j] += of.x; g[2 * j + 1] += of.y;
-            }
-          }
-          uint4 o;
-          o.x = Op16<T16>::pack(g[0], g[1]); o.y = Op16<T16>::pack(g[2], g[3]);
-          o.z = Op16<T16>::pack(g[4], g[5]); o.w = Op16<T16>::pack(g[6], g[7]);
-          reinterpret_cast<uint4*>(op)[c] = o;
-        }
+        __syncwarp();
       }
     }
-    tc_fence_before();
-    __syncthreads();
   }
 
-  // ---- dQ partial of this range: latent block wg by thread group wg -----------------------------
-  if (!aborted && wg < n_mblk) {
-    uint32_t r[D];
-    if constexpr (D == 16) tmem_ld16(lane_base + cDQ + 32 * wg, r);
-    else tmem_ld32(lane_base + cDQ + 32 * wg, r);
-    tmem_wait_ld();
-    const int m = wg * 128 + row;
-    if (m < M) {
-      float* o = dq_out + (long long)m * D;
+  // ---- the last tile's dV/dK, and the dQ partial of this range ----------------------------------
+  if (!aborted) {
+    mbar_wait(bar_mma, ph_mma, a.status, abort_flag);
+    tc_fence_after();
+    store_tile(n_tiles - 1);
+    if (cg < n_mblk) {
+      uint32_t r[D];
+      if constexpr (D == 16) tmem_ld16(lane_base + cDQ + D * cg, r);
+      else tmem_ld32(lane_base + cDQ + D * cg, r);
+      tmem_wait_ld();
+      const int m = cg * 128 + row;
+      if (m < M) {
+        float* o = dq_out + (long long)m * D;
 #pragma unroll
-      for (int c = 0; c < D / 4; ++c)
-        reinterpret_cast<float4*>(o)[c] = make_float4(__uint_as_float(r[4 * c]) * a.scale, __uint_as_float(r[4 * c + 1]) * a.scale,
-                                                      __uint_as_float(r[4 * c + 2]) * a.scale, __uint_as_float(r[4 * c + 3]) * a.scale);
+        for (int c = 0; c < D / 4; ++c)
+          reinterpret_cast<float4*>(o)[c] = make_float4(__uint_as_float(r[4 * c]) * a.scale, __uint_as_float(r[4 * c + 1]) * a.scale,
+                                                        __uint_as_float(r[4 * c + 2]) * a.scale, __uint_as_float(r[4 * c + 3]) * a.scale);
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc<512>(tmem);
+  if (warp == 0) tmem_dealloc<BwdShape<D>::kCols>(tmem);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -433,9 +475,12 @@ static int launch_bwd(const Ctx& c, const void* q, const void* k, const void* v,
   a.status = tc_status_ptr();
   a.flag = flag;
   constexpr int smem = BwdSmem<D>::kBytes;
-  if (tc_set_dyn_smem(reinterpret_cast<const void*>(&k_tc_bwd<D, T16, false>), smem) != FLARE_OK ||
-      tc_set_dyn_smem(reinterpret_cast<const void*>(&k_tc_bwd<D, T16, true>), smem) != FLARE_OK)
-    return FLARE_ECUDA;
+  using Kernel = decltype(&k_tc_bwd<D, T16, false, true>);
+  const bool plain = use_g && use_s && !a.drop.on;
+  const Kernel first = plain ? &k_tc_bwd<D, T16, false, true> : &k_tc_bwd<D, T16, false, false>;
+  const Kernel later = plain ? &k_tc_bwd<D, T16, true, true> : &k_tc_bwd<D, T16, true, false>;
+  for (Kernel k : {first, later})
+    if (tc_set_dyn_smem(reinterpret_cast<const void*>(k), smem) != FLARE_OK) return FLARE_ECUDA;
   const long long grid = (long long)c.n_splits * c.B * c.H;
   if (grid > 0x7fffffffLL) return FLARE_EUNSUPPORTED;
   for (int m0 = 0; m0 < c.M; m0 += 256) {
@@ -446,8 +491,7 @@ static int launch_bwd(const Ctx& c, const void* q, const void* k, const void* v,
                        (qb ? c.qs[0] : c.qs[1] * c.H) * e, 256))
       return FLARE_EUNSUPPORTED;
     a.M = mb; a.m0 = m0;
-    if (m0 == 0) launch_dep(k_tc_bwd<D, T16, false>, dim3((unsigned)grid), dim3(256), smem, st, tmQ, tmK, tmV, tmG, tmY, a);
-    else launch_dep(k_tc_bwd<D, T16, true>, dim3((unsigned)grid), dim3(256), smem, st, tmQ, tmK, tmV, tmG, tmY, a);
+    launch_dep(m0 == 0 ? first : later, dim3((unsigned)grid), dim3(BwdShape<D>::kThreads), smem, st, tmQ, tmK, tmV, tmG, tmY, a);
   }
   return FLARE_OK;
 }

@@ -398,3 +398,50 @@ def test_qk_norm_and_output_gate_variants(fb, cuda_dev):
     assert abs(a[0] - b[0]) <= 1e-5 * abs(b[0])
     for u, w in zip(a[1:], b[1:]):
         assert O.rel_l2(u.cpu(), w.cpu()) <= 1e-4
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
+@pytest.mark.parametrize("B,H,N,M,D", [
+    (1, 1, 1, 1, 8),            # one row: three of the four warps of a block have nothing
+    (1, 2, 127, 33, 8),         # a second row per lane half used
+    (2, 1, 129, 65, 16),        # a third, and a token tile of one
+    (1, 1, 300, 260, 8),        # more latents than one staged tile
+    (1, 8, 5000, 130, 8),       # enough blocks for four rows per lane, the last block of latents nearly empty
+    (1, 8, 5000, 96, 16),
+    (2, 4, 3001, 80, 32),
+])
+def test_register_blocked_fp32_kernels(fb, cuda_dev, dtype, tol, B, H, N, M, D):
+    """Rows per lane, token quarters and their merge, with a key mask that empties whole tiles.  bf16 results are
+    rounded to 2^-9 and delta is taken from the rounded y; fp32 ones differ by the order of the sums."""
+    q, k, v, dy = O.make_inputs(B, H, N, M, D, dtype=dtype, seed=N + M)
+    mask = torch.rand(B, N, generator=torch.Generator().manual_seed(3)) < 0.7
+    mask[:, 128:N // 2] = False
+    mask[:, 0] = True
+    prev = fb.set_kernel_path("simt")
+    try:
+        got = run_mixer(fb, q, k, v, dy, 0.7, cuda_dev, key_mask=mask)
+    finally:
+        fb.set_kernel_path(prev)
+    qf, kf, vf = (t.double().requires_grad_(True) for t in (q, k, v))
+    y = O.mixer_lra(qf, kf, vf, 0.7, mask)
+    y.backward(dy.double())
+    ref = [y.detach(), qf.grad, kf.grad, vf.grad]
+    if N == 1:                  # one token: dq and dk vanish
+        got, ref = [got[0], got[3]], [ref[0], ref[3]]
+    assert_close([g.double() for g in got], ref, tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,M", [(129, 32), (1000, 64), (640, 96), (257, 160), (1500, 256), (700, 320)])
+def test_general_backward_in_64_latent_steps(fb, cuda_dev, dtype, N, M):
+    """D = 16: steps of 64 latents, dQ per pair of steps; half-filled steps and pairs, ragged tiles, a mask."""
+    B, H, D = 2, 3, 16
+    q, k, v, dy = O.make_inputs(B, H, N, M, D, dtype=dtype, seed=N + M)
+    mask = torch.rand(B, N, generator=torch.Generator().manual_seed(5)) < 0.8
+    got = run_mixer(fb, q, k, v, dy, 1.0, cuda_dev, key_mask=mask)
+    assert fb.device_status() == 0
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    y = O.mixer_lra(qf, kf, vf, 1.0, mask)
+    y.backward(dy.float())
+    # two correct 16-bit evaluations differ by a few roundings of the operands (bf16: 2^-9 each)
+    assert_close(got, [y.detach(), qf.grad, kf.grad, vf.grad], 1e-2 if dtype == torch.bfloat16 else 2e-3)
