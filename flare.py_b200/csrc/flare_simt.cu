@@ -412,6 +412,543 @@ k_bwd_tokens(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* _
 }
 
 // ---------------------------------------------------------------------------------
+// Register-blocked forms of the five passes for small head dims (D <= 32; the two widest passes D <= 16).
+//
+// With one row per thread every fused multiply-add pair costs a shared-memory load (a broadcast LDS.128 feeds four
+// of them), and the load pipe, not the FMA pipe, bounds the kernel: 13 clocks per SM and warp of scores at D = 8
+// where the arithmetic needs 4.  Here a lane owns R rows (latents or tokens), so that one load feeds R rows, and
+// the products are packed two-wide (fma.rn.f32x2).  The four warps of a block share the same 32 R rows and take a
+// quarter of every staged tile each, their partial sums meeting once at the end in fixed order: the grid stays as
+// fine as with one row per thread, and small M no longer leaves threads idle (32 R is chosen not to exceed M by more
+// than one power of two).
+// R is what the registers hold: R * D * (operands + accumulators) <= 160 floats.  Measured, one row per thread against
+// these: N = 500 000, H = 8, M = 512, D = 8 bf16: gather 3.03 -> 1.82 ms, scatter 2.33 -> 1.89, dZ 2.93 -> 1.54, tokens
+// 7.23 -> 4.80, dQ 8.19 -> 4.71; B = 2, H = 8, N = 4096, M = 64, D = 16 fp32: dQ 98 -> 33 us, gather 36 -> 18, dZ 41 -> 21.
+// ---------------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ float dot2(const float2* a, const float2* b) {
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) s = __ffma2_rn(a[i], b[i], s);
+  return s.x + s.y;
+}
+template <int D>
+__device__ __forceinline__ void axpy2(float2* acc, float w, const float2* x) {
+  const float2 w2 = make_float2(w, w);
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) acc[i] = __ffma2_rn(w2, x[i], acc[i]);
+}
+template <int D>
+__device__ __forceinline__ void row_from_smem(float2* r, const float* sm) {
+#pragma unroll
+  for (int i = 0; i < D / 4; ++i) {
+    const float4 t = reinterpret_cast<const float4*>(sm)[i];
+    r[2 * i] = make_float2(t.x, t.y);
+    r[2 * i + 1] = make_float2(t.z, t.w);
+  }
+}
+template <typename T, int D>
+__device__ __forceinline__ void row_from_global(float2* r, const T* p, float f) {
+  float t[D];
+  load_f32<T, D>(p, t);
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) r[i] = make_float2(t[2 * i] * f, t[2 * i + 1] * f);
+}
+template <int D>
+__device__ __forceinline__ void zero_row(float2* r) {
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) r[i] = make_float2(0.f, 0.f);
+}
+// The part [lo, hi) of `cnt` staged rows that warp w of four takes: whole groups of G rows.
+template <int G>
+__device__ __forceinline__ void quarter(int cnt, int w, int& lo, int& hi) {
+  const int per = ((cnt + 4 * G - 1) / (4 * G)) * G;
+  lo = min(cnt, w * per);
+  hi = min(cnt, lo + per);
+}
+template <int D> struct TileR { static constexpr int v = D <= 16 ? 128 : 64; };   // staged tokens of a latent-row pass
+
+template <typename T, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+k_gather_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+              const uint8_t* __restrict__ mask, float* __restrict__ rec) {
+  constexpr int LPB = 32 * R, TN = TileR<D>::v, W = D + 2;
+  constexpr int kStage = 2 * TN * D + TN, kMerge = 4 * LPB * W;
+  __shared__ __align__(16) float sm[kStage > kMerge ? kStage : kMerge];
+  float* sK = sm;
+  float* sV = sK + TN * D;
+  float* sKeep = sV + TN * D;
+  const int split = blockIdx.x, bh = blockIdx.z, b = bh / c.H, h = bh % c.H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lat0 = blockIdx.y * LPB + lane;
+  float2 qr[R][D / 2], acc[R][D / 2];
+  float mx[R], l[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    zero_row<D>(qr[r]); zero_row<D>(acc[r]);
+    mx[r] = -INFINITY; l[r] = 0.f;
+    const int lat = lat0 + 32 * r;
+    if (lat < c.M) row_from_global<T, D>(qr[r], q + b * c.qs[0] + h * c.qs[1] + (long long)lat * c.qs[2], c.scale * kLog2e);
+  }
+  const int n0 = split * c.chunk, n1 = min(c.N, n0 + c.chunk);
+  const T* kb = k + b * c.ks[0] + h * c.ks[1];
+  const T* vb = v + b * c.vs[0] + h * c.vs[1];
+  for (int t0 = n0; t0 < n1; t0 += TN) {
+    const int cnt = min(TN, n1 - t0);
+    __syncthreads();
+    stage_rows<T, D>(sK, kb + (long long)t0 * c.ks[2], c.ks[2], cnt, TN);
+    stage_rows<T, D>(sV, vb + (long long)t0 * c.vs[2], c.vs[2], cnt, TN);
+    for (int i = threadIdx.x; i < TN; i += kThreads)
+      sKeep[i] = (i < cnt && (!mask || mask[(long long)b * c.N + t0 + i])) ? 1.f : 0.f;
+    __syncthreads();
+    int lo, hi;
+    quarter<4>(cnt, warp, lo, hi);                 // groups of 4 stay inside the TN staged rows; rows past cnt have keep 0
+    for (int j0 = lo; j0 < hi; j0 += 4) {
+      float s[4][R];
+      bool grow = false;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        float2 kr[D / 2];
+        row_from_smem<D>(kr, sK + (j0 + jj) * D);
+        const bool keep = sKeep[j0 + jj] != 0.f;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float d = dot2<D>(qr[r], kr);
+          s[jj][r] = keep ? d : -INFINITY;
+          grow |= s[jj][r] > mx[r];
+        }
+      }
+      if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float mnew = fmaxf(fmaxf(mx[r], fmaxf(s[0][r], s[1][r])), fmaxf(s[2][r], s[3][r]));
+          const float corr = mnew == -INFINITY ? 1.f : exp2f(mx[r] - mnew);
+          l[r] *= corr;
+#pragma unroll
+          for (int i = 0; i < D / 2; ++i) { acc[r][i].x *= corr; acc[r][i].y *= corr; }
+          mx[r] = mnew;
+        }
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        float2 vr[D / 2];
+        row_from_smem<D>(vr, sV + (j0 + jj) * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float p = exp2f(s[jj][r] - (mx[r] == -INFINITY ? 0.f : mx[r]));
+          l[r] += p;
+          axpy2<D>(acc[r], p, vr);
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float* o = sm + (warp * LPB + 32 * r + lane) * W;
+#pragma unroll
+    for (int i = 0; i < D / 2; ++i) { o[2 * i] = acc[r][i].x; o[2 * i + 1] = acc[r][i].y; }
+    o[D] = mx[r]; o[D + 1] = l[r];
+  }
+  __syncthreads();
+  const int lat = blockIdx.y * LPB + threadIdx.x;
+  if (threadIdx.x < LPB && lat < c.M) {
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) m = fmaxf(m, sm[(w * LPB + threadIdx.x) * W + D]);
+    float tot[D + 1];
+#pragma unroll
+    for (int i = 0; i <= D; ++i) tot[i] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float* o = sm + (w * LPB + threadIdx.x) * W;
+      const float f = o[D] == -INFINITY ? 0.f : exp2f(o[D] - m);
+      // (a part whose rows were all excluded holds zeros)
+#pragma unroll
+      for (int i = 0; i < D; ++i) tot[i] = fmaf(f, o[i], tot[i]);
+      tot[D] = fmaf(f, o[D + 1], tot[D]);
+    }
+    float* o = rec + ((((long long)split * c.B + b) * c.H + h) * c.M + lat) * W;
+#pragma unroll
+    for (int i = 0; i < D; ++i) o[i] = tot[i];
+    o[D] = m * kLn2; o[D + 1] = tot[D];
+  }
+}
+
+// Sum over the four warps of NV floats per row (each warp's rows 32 r + lane), result handed to thread = row.
+template <int NV, int R>
+__device__ __forceinline__ void merge_rows(float* sm, const float2 (&acc)[R][NV / 2], float* tot) {
+  constexpr int LPB = 32 * R;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float* o = sm + (warp * LPB + 32 * r + lane) * (NV + 1);
+#pragma unroll
+    for (int i = 0; i < NV / 2; ++i) { o[2 * i] = acc[r][i].x; o[2 * i + 1] = acc[r][i].y; }
+  }
+  __syncthreads();
+  if (threadIdx.x < LPB) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float a = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) a += sm[(w * LPB + threadIdx.x) * (NV + 1) + i];
+      tot[i] = a;
+    }
+  }
+}
+
+template <typename T, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+k_dz_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ dy,
+          const uint8_t* __restrict__ mask, const float* __restrict__ lse_n, float* __restrict__ dz_part) {
+  constexpr int LPB = 32 * R, TN = TileR<D>::v;
+  constexpr int kStage = 2 * TN * D + TN, kMerge = 4 * LPB * (D + 1);
+  __shared__ __align__(16) float sm[kStage > kMerge ? kStage : kMerge];
+  float* sK = sm;
+  float* sG = sK + TN * D;
+  float* sC2 = sG + TN * D;
+  const int split = blockIdx.x, bh = blockIdx.z, b = bh / c.H, h = bh % c.H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lat0 = blockIdx.y * LPB + lane;
+  float2 qr[R][D / 2], acc[R][D / 2];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    zero_row<D>(qr[r]); zero_row<D>(acc[r]);
+    const int lat = lat0 + 32 * r;
+    if (lat < c.M) row_from_global<T, D>(qr[r], q + b * c.qs[0] + h * c.qs[1] + (long long)lat * c.qs[2], c.scale * kLog2e);
+  }
+  const int n0 = split * c.chunk, n1 = min(c.N, n0 + c.chunk);
+  const T* kb = k + b * c.ks[0] + h * c.ks[1];
+  const T* gb = dy + b * c.dys[0] + h * c.dys[1];
+  const float* cb = lse_n + ((long long)b * c.H + h) * c.N;
+  for (int t0 = n0; t0 < n1; t0 += TN) {
+    const int cnt = min(TN, n1 - t0);
+    __syncthreads();
+    stage_rows<T, D>(sK, kb + (long long)t0 * c.ks[2], c.ks[2], cnt, TN);
+    stage_rows<T, D>(sG, gb + (long long)t0 * c.dys[2], c.dys[2], cnt, TN);
+    for (int i = threadIdx.x; i < TN; i += kThreads) {
+      const bool keep = i < cnt && (!mask || mask[(long long)b * c.N + t0 + i]);
+      sC2[i] = keep ? cb[t0 + i] * kLog2e : INFINITY;      // +inf => weight 0
+    }
+    __syncthreads();
+    int lo, hi;
+    quarter<2>(cnt, warp, lo, hi);
+#pragma unroll 2
+    for (int j = lo; j < hi; ++j) {
+      float2 kr[D / 2], gr[D / 2];
+      row_from_smem<D>(kr, sK + j * D);
+      row_from_smem<D>(gr, sG + j * D);
+      const float c2 = sC2[j];
+#pragma unroll
+      for (int r = 0; r < R; ++r) axpy2<D>(acc[r], exp2f(dot2<D>(qr[r], kr) - c2), gr);
+    }
+  }
+  float tot[D];
+  merge_rows<D, R>(sm, acc, tot);
+  const int lat = blockIdx.y * LPB + threadIdx.x;
+  if (threadIdx.x < LPB && lat < c.M) {
+    float* o = dz_part + ((((long long)split * c.B + b) * c.H + h) * c.M + lat) * D;
+#pragma unroll
+    for (int i = 0; i < D; ++i) o[i] = tot[i];
+  }
+}
+
+template <typename T, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+k_dq_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ dy,
+          const uint8_t* __restrict__ mask, const float* __restrict__ z32, const float* __restrict__ dz32,
+          const float* __restrict__ lse_m, const float* __restrict__ lse_n, const float* __restrict__ delta_n,
+          float* __restrict__ dq_part) {
+  constexpr int LPB = 32 * R, TN = TileR<D>::v;
+  constexpr int kStage = 3 * TN * D + 2 * TN, kMerge = 4 * LPB * (D + 1);
+  __shared__ __align__(16) float sm[kStage > kMerge ? kStage : kMerge];
+  float* sK = sm;
+  float* sV = sK + TN * D;
+  float* sG = sV + TN * D;
+  float* sC2 = sG + TN * D;
+  float* sDel = sC2 + TN;
+  const bool use_g = (c.terms & FLARE_TERM_GATHER) != 0, use_s = (c.terms & FLARE_TERM_SCATTER) != 0;
+  const int split = blockIdx.x, bh = blockIdx.z, b = bh / c.H, h = bh % c.H;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lat0 = blockIdx.y * LPB + lane;
+  float2 qr[R][D / 2], zr[R][D / 2], dzr[R][D / 2], acc[R][D / 2];
+  float L2[R], Delta[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    zero_row<D>(qr[r]); zero_row<D>(zr[r]); zero_row<D>(dzr[r]); zero_row<D>(acc[r]);
+    L2[r] = INFINITY; Delta[r] = 0.f;
+    const int lat = lat0 + 32 * r;
+    if (lat < c.M) {
+      const long long row = ((long long)b * c.H + h) * c.M + lat;
+      row_from_global<T, D>(qr[r], q + b * c.qs[0] + h * c.qs[1] + (long long)lat * c.qs[2], c.scale * kLog2e);
+      row_from_global<float, D>(zr[r], z32 + row * D, 1.f);
+      if (use_g) {
+        row_from_global<float, D>(dzr[r], dz32 + row * D, 1.f);
+        Delta[r] = dot2<D>(dzr[r], zr[r]);
+        L2[r] = lse_m[row] * kLog2e;
+      }
+    }
+  }
+  const int n0 = split * c.chunk, n1 = min(c.N, n0 + c.chunk);
+  const T* kb = k + b * c.ks[0] + h * c.ks[1];
+  const T* vb = use_g ? v + b * c.vs[0] + h * c.vs[1] : nullptr;
+  const T* gb = use_s ? dy + b * c.dys[0] + h * c.dys[1] : nullptr;
+  const long long tokrow = ((long long)b * c.H + h) * c.N;
+  for (int t0 = n0; t0 < n1; t0 += TN) {
+    const int cnt = min(TN, n1 - t0);
+    __syncthreads();
+    stage_rows<T, D>(sK, kb + (long long)t0 * c.ks[2], c.ks[2], cnt, TN);
+    if (use_g) stage_rows<T, D>(sV, vb + (long long)t0 * c.vs[2], c.vs[2], cnt, TN);
+    if (use_s) stage_rows<T, D>(sG, gb + (long long)t0 * c.dys[2], c.dys[2], cnt, TN);
+    for (int i = threadIdx.x; i < TN; i += kThreads) {
+      const bool keep = i < cnt && (!mask || mask[(long long)b * c.N + t0 + i]);
+      sC2[i] = !keep ? -INFINITY : use_s ? lse_n[tokrow + t0 + i] * kLog2e : INFINITY;   // -inf: skip this token
+      sDel[i] = (keep && use_s) ? delta_n[tokrow + t0 + i] : 0.f;
+    }
+    __syncthreads();
+    int lo, hi;
+    quarter<1>(cnt, warp, lo, hi);
+    for (int j = lo; j < hi; ++j) {
+      const float c2 = sC2[j];
+      if (c2 == -INFINITY) continue;               // the same for the whole warp
+      float2 kr[D / 2], x[D / 2];
+      float dS[R], s[R];
+      row_from_smem<D>(kr, sK + j * D);
+#pragma unroll
+      for (int r = 0; r < R; ++r) { s[r] = dot2<D>(qr[r], kr); dS[r] = 0.f; }
+      if (use_g) {
+        row_from_smem<D>(x, sV + j * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) dS[r] = exp2f(s[r] - L2[r]) * (dot2<D>(dzr[r], x) - Delta[r]);
+      }
+      if (use_s) {
+        row_from_smem<D>(x, sG + j * D);
+        const float del = sDel[j];
+#pragma unroll
+        for (int r = 0; r < R; ++r) dS[r] = fmaf(exp2f(s[r] - c2), dot2<D>(zr[r], x) - del, dS[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) axpy2<D>(acc[r], dS[r], kr);
+    }
+  }
+  float tot[D];
+  merge_rows<D, R>(sm, acc, tot);
+  const int lat = blockIdx.y * LPB + threadIdx.x;
+  if (threadIdx.x < LPB && lat < c.M) {
+    float* o = dq_part + ((((long long)split * c.B + b) * c.H + h) * c.M + lat) * D;
+#pragma unroll
+    for (int i = 0; i < D; ++i) o[i] = tot[i] * c.scale;
+  }
+}
+
+template <typename T, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+k_scatter_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ z32,
+               const uint8_t* __restrict__ mask, T* __restrict__ y, float* __restrict__ lse_n) {
+  constexpr int TPB = 32 * R, MC = 2048 / D, W = D + 2;
+  constexpr int kStage = 2 * MC * D, kMerge = 4 * TPB * W;
+  __shared__ __align__(16) float sm[kStage > kMerge ? kStage : kMerge];
+  float* sQ = sm;
+  float* sZ = sQ + MC * D;
+  const int b = blockIdx.z, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float2 kr[R][D / 2], acc[R][D / 2];
+  float mx[R], l[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    zero_row<D>(kr[r]); zero_row<D>(acc[r]);
+    mx[r] = -INFINITY; l[r] = 0.f;
+    const int tok = blockIdx.x * TPB + 32 * r + lane;
+    if (tok < c.N) row_from_global<T, D>(kr[r], k + b * c.ks[0] + h * c.ks[1] + (long long)tok * c.ks[2], 1.f);
+  }
+  const T* qb = q + b * c.qs[0] + h * c.qs[1];
+  const float* zb = z32 + ((long long)b * c.H + h) * c.M * D;
+  const float f = c.scale * kLog2e;
+  for (int m0 = 0; m0 < c.M; m0 += MC) {
+    const int cnt = min(MC, c.M - m0);
+    __syncthreads();
+    stage_rows<T, D>(sQ, qb + (long long)m0 * c.qs[2], c.qs[2], cnt, MC);
+    stage_rows<float, D>(sZ, zb + (long long)m0 * D, D, cnt, MC);
+    __syncthreads();
+    int lo, hi;
+    quarter<4>(cnt, warp, lo, hi);
+    for (int j0 = lo; j0 < hi; j0 += 4) {
+      float s[4][R];
+      bool grow = false;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        float2 qr[D / 2];
+        row_from_smem<D>(qr, sQ + (j0 + jj) * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float d = dot2<D>(kr[r], qr) * f;
+          s[jj][r] = (j0 + jj < cnt) ? d : -INFINITY;
+          grow |= s[jj][r] > mx[r];
+        }
+      }
+      if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float mnew = fmaxf(fmaxf(mx[r], fmaxf(s[0][r], s[1][r])), fmaxf(s[2][r], s[3][r]));
+          const float corr = exp2f(mx[r] - mnew);
+          l[r] *= corr;
+#pragma unroll
+          for (int i = 0; i < D / 2; ++i) { acc[r][i].x *= corr; acc[r][i].y *= corr; }
+          mx[r] = mnew;
+        }
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        float2 zr[D / 2];
+        row_from_smem<D>(zr, sZ + (j0 + jj) * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float p = exp2f(s[jj][r] - mx[r]);
+          l[r] += p;
+          axpy2<D>(acc[r], p, zr);
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float* o = sm + (warp * TPB + 32 * r + lane) * W;
+#pragma unroll
+    for (int i = 0; i < D / 2; ++i) { o[2 * i] = acc[r][i].x; o[2 * i + 1] = acc[r][i].y; }
+    o[D] = mx[r]; o[D + 1] = l[r];
+  }
+  __syncthreads();
+  const int tok = blockIdx.x * TPB + threadIdx.x;
+  if (threadIdx.x < TPB && tok < c.N) {
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) m = fmaxf(m, sm[(w * TPB + threadIdx.x) * W + D]);
+    float tot[D], ls = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) tot[i] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float* o = sm + (w * TPB + threadIdx.x) * W;
+      const float e = o[D] == -INFINITY ? 0.f : exp2f(o[D] - m);      // a warp without latents
+#pragma unroll
+      for (int i = 0; i < D; ++i) tot[i] = fmaf(e, o[i], tot[i]);
+      ls = fmaf(e, o[D + 1], ls);
+    }
+    const bool keep = !mask || mask[(long long)b * c.N + tok];
+    const float inv = keep ? 1.f / ls : 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) tot[i] *= inv;
+    store_from_f32<T, D>(y + b * c.ys[0] + h * c.ys[1] + (long long)tok * c.ys[2], tot);
+    if (lse_n) lse_n[((long long)b * c.H + h) * c.N + tok] = (m + log2f(ls)) * kLn2;
+  }
+}
+
+template <typename T, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+k_bwd_tokens_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                  const T* __restrict__ dy, const T* __restrict__ y, const uint8_t* __restrict__ mask,
+                  const float* __restrict__ z32, const float* __restrict__ dz32, const float* __restrict__ lse_m,
+                  const float* __restrict__ lse_n, T* __restrict__ dk, T* __restrict__ dv, float* __restrict__ delta_n) {
+  constexpr int TPB = 32 * R, MC = 2048 / D;
+  constexpr int kStage = 3 * MC * D + 2 * MC, kMerge = 4 * TPB * (2 * D + 1);
+  __shared__ __align__(16) float sm[kStage > kMerge ? kStage : kMerge];
+  float* sQ = sm;
+  float* sZ = sQ + MC * D;
+  float* sDZ = sZ + MC * D;
+  float2* sLD = reinterpret_cast<float2*>(sDZ + MC * D);            // {L_m log2e, Delta_m}
+  const bool use_g = (c.terms & FLARE_TERM_GATHER) != 0, use_s = (c.terms & FLARE_TERM_SCATTER) != 0;
+  const int b = blockIdx.z, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float2 kr[R][D / 2], vr[R][D / 2], gr[R][D / 2], acc[R][D];       // acc: dk | dv
+  float delta[R], C2[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    zero_row<D>(kr[r]); zero_row<D>(vr[r]); zero_row<D>(gr[r]); zero_row<2 * D>(acc[r]);
+    delta[r] = 0.f; C2[r] = INFINITY;
+    const int tok = blockIdx.x * TPB + 32 * r + lane;
+    if (tok < c.N && (!mask || mask[(long long)b * c.N + tok])) {
+      const long long t = tok;
+      row_from_global<T, D>(kr[r], k + b * c.ks[0] + h * c.ks[1] + t * c.ks[2], 1.f);
+      if (use_g) row_from_global<T, D>(vr[r], v + b * c.vs[0] + h * c.vs[1] + t * c.vs[2], 1.f);
+      if (use_s) {
+        row_from_global<T, D>(gr[r], dy + b * c.dys[0] + h * c.dys[1] + t * c.dys[2], 1.f);
+        float2 yr[D / 2];
+        row_from_global<T, D>(yr, y + b * c.ys[0] + h * c.ys[1] + t * c.ys[2], 1.f);
+        delta[r] = dot2<D>(gr[r], yr);
+        C2[r] = lse_n[((long long)b * c.H + h) * c.N + tok] * kLog2e;
+      }
+    }
+  }
+  const T* qb = q + b * c.qs[0] + h * c.qs[1];
+  const long long latrow = ((long long)b * c.H + h) * c.M;
+  const float f = c.scale * kLog2e;
+  for (int m0 = 0; m0 < c.M; m0 += MC) {
+    const int cnt = min(MC, c.M - m0);
+    __syncthreads();
+    stage_rows<T, D>(sQ, qb + (long long)m0 * c.qs[2], c.qs[2], cnt, MC);
+    stage_rows<float, D>(sZ, z32 + (latrow + m0) * D, D, cnt, MC);
+    if (use_g) stage_rows<float, D>(sDZ, dz32 + (latrow + m0) * D, D, cnt, MC);
+    __syncthreads();
+    for (int r = threadIdx.x; r < MC; r += kThreads) {
+      float d = 0.f, l2 = INFINITY;
+      if (use_g && r < cnt) {
+        float2 a[D / 2], z[D / 2];
+        row_from_smem<D>(a, sDZ + r * D);
+        row_from_smem<D>(z, sZ + r * D);
+        d = dot2<D>(a, z);
+        l2 = lse_m[latrow + m0 + r] * kLog2e;
+      }
+      sLD[r] = make_float2(l2, d);
+    }
+    __syncthreads();
+    int lo, hi;
+    quarter<1>(cnt, warp, lo, hi);
+    for (int j = lo; j < hi; ++j) {
+      float2 qr[D / 2], x[D / 2];
+      float s[R], dS[R];
+      row_from_smem<D>(qr, sQ + j * D);
+#pragma unroll
+      for (int r = 0; r < R; ++r) { s[r] = dot2<D>(kr[r], qr) * f; dS[r] = 0.f; }
+      if (use_g) {
+        const float2 ld = sLD[j];
+        row_from_smem<D>(x, sDZ + j * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float P = exp2f(s[r] - ld.x);
+          dS[r] = P * (dot2<D>(vr[r], x) - ld.y);
+          axpy2<D>(acc[r] + D / 2, P, x);
+        }
+      }
+      if (use_s) {
+        row_from_smem<D>(x, sZ + j * D);
+#pragma unroll
+        for (int r = 0; r < R; ++r) dS[r] = fmaf(exp2f(s[r] - C2[r]), dot2<D>(gr[r], x) - delta[r], dS[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) axpy2<D>(acc[r], dS[r], qr);
+    }
+  }
+  float tot[2 * D];
+  merge_rows<2 * D, R>(sm, acc, tot);
+  // delta of a row sits in the lane that owns it, in every warp alike
+  if (delta_n && warp == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int tok = blockIdx.x * TPB + 32 * r + lane;
+      if (tok < c.N) delta_n[((long long)b * c.H + h) * c.N + tok] = delta[r];
+    }
+  }
+  const int tok = blockIdx.x * TPB + threadIdx.x;
+  if (threadIdx.x < TPB && tok < c.N) {
+    const bool keep = !mask || mask[(long long)b * c.N + tok];
+#pragma unroll
+    for (int i = 0; i < D; ++i) { tot[i] = keep ? tot[i] * c.scale : 0.f; tot[D + i] = keep ? tot[D + i] : 0.f; }
+    store_from_f32<T, D>(dk + b * c.dks[0] + h * c.dks[1] + (long long)tok * c.dks[2], tot);
+    if (use_g) store_from_f32<T, D>(dv + b * c.dvs[0] + h * c.dvs[1] + (long long)tok * c.dvs[2], tot + D);
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // log-sum-exp combine of records, and plain ordered sum
 // ---------------------------------------------------------------------------------
 // Where part p of a partial array lives: at base + p * stride (one buffer of this GPU), or at ptrs[p]
@@ -430,7 +967,9 @@ struct PartsPtrs {
 // accumulator rows are in flight.  The kernel's time is the latency of its dependent loads, not their volume:
 // three rounds of loads instead of one per part.  The order of every sum is fixed (shuffle tree over the
 // lanes, then ascending parts), so equal inputs give equal bits on every rank.
-template <typename Parts>
+// NI: column groups of 32 (D <= 32 NI); JB: parts whose rows are in flight together -- with the 64 predicated loads
+// of NI = 4, JB = 16 for every row, one part per row (B H = 256, M = 128, D = 16) took 40 us for 2.4 MB.
+template <int NI, int JB, typename Parts>
 __global__ void __launch_bounds__(kThreads)
 k_combine(Parts parts, int n_parts, long long rows, int D, int dtype,
           float* __restrict__ z32, void* __restrict__ z_out, float* __restrict__ lse_m,
@@ -448,7 +987,9 @@ k_combine(Parts parts, int n_parts, long long rows, int D, int dtype,
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float lt = 0.f;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};             // d = lane, lane + 32, ... (D <= 128)
+  float acc[NI];                                   // d = lane, lane + 32, ...
+#pragma unroll
+  for (int i = 0; i < NI; ++i) acc[i] = 0.f;
   for (int p0 = 0; p0 < n_parts; p0 += 32) {
     const int p = p0 + lane;
     float w = 0.f, wl = 0.f;
@@ -461,25 +1002,25 @@ k_combine(Parts parts, int n_parts, long long rows, int D, int dtype,
     for (int o = 16; o > 0; o >>= 1) wl += __shfl_xor_sync(0xffffffffu, wl, o);
     lt += wl;
     const int cnt = min(32, n_parts - p0);
-    for (int j0 = 0; j0 < cnt; j0 += 16) {
-      float av[16][4];
+    for (int j0 = 0; j0 < cnt; j0 += JB) {
+      float av[JB][NI];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < JB; ++j) {
         const float* src = parts.at(p0 + min(j0 + j, cnt - 1)) + row * W;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) av[j][i] = (j0 + j < cnt && lane + 32 * i < D) ? src[lane + 32 * i] : 0.f;
+        for (int i = 0; i < NI; ++i) av[j][i] = (j0 + j < cnt && lane + 32 * i < D) ? src[lane + 32 * i] : 0.f;
       }
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < JB; ++j) {
         const float wj = __shfl_sync(0xffffffffu, w, (j0 + j) & 31);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] = fmaf(wj, av[j][i], acc[i]);
+        for (int i = 0; i < NI; ++i) acc[i] = fmaf(wj, av[j][i], acc[i]);
       }
     }
   }
   const float inv = 1.f / lt;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < NI; ++i) {
     const int d = lane + 32 * i;
     if (d < D) {
       if (rec_out) rec_out[row * W + d] = acc[i];
@@ -554,18 +1095,39 @@ static inline dim3 tok_grid(const Ctx& c) {
   const int tpb = kThreads / tpt;
   return dim3((c.N + tpb - 1) / tpb, c.H, c.B);
 }
+// Rows per lane of the register-blocked kernels (0: one row per thread is the better form -- wide rows, whose
+// operands leave no registers for a second one).  kArrays: D-wide register arrays per row.
+template <int D, int kArrays> constexpr int max_rows() {
+  return 4 * D * kArrays <= 160 ? 4 : 2 * D * kArrays <= 160 ? 2 : 0;
+}
+// Launch with R rows per lane, R <= RM: no more than the rows fill (a block takes 32 R of them), and no more than
+// leaves one and a half blocks per SM (`others_` blocks run per block of rows).
+#define FLARE_ROWS(RM_, rows_, others_, ...)                                     \
+  if constexpr (RM_ > 0) {                                                       \
+    const long long r32 = ((rows_) + 31) / 32, least = 3LL * num_sms() / 2;          \
+    if (RM_ >= 4 && r32 > 2 && (r32 + 3) / 4 * (others_) >= least) { constexpr int kR = RM_ >= 4 ? 4 : 1; __VA_ARGS__; } \
+    else if (r32 > 1 && (r32 + 1) / 2 * (others_) >= least) { constexpr int kR = 2; __VA_ARGS__; } \
+    else                          { constexpr int kR = 1; __VA_ARGS__; }         \
+    return FLARE_OK;                                                             \
+  }
 
 int simt_gather_partial(const Ctx& c, int dtype, const void* q, const void* k, const void* v,
                         const uint8_t* mask, float* rec, cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    k_gather_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, mask, rec)));
+    constexpr int RM = max_rows<kD, 2>();
+    FLARE_ROWS(RM, c.M, (long long)c.n_splits * c.B * c.H, k_gather_rows<T, kD, kR><<<dim3(c.n_splits, (c.M + 32 * kR - 1) / (32 * kR), c.B * c.H), kThreads, 0, st>>>(
+                            c, (const T*)q, (const T*)k, (const T*)v, mask, rec))
+    else k_gather_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, mask, rec)));
   return FLARE_OK;
 }
 
 int simt_dz_partial(const Ctx& c, int dtype, const void* q, const void* k, const void* dy,
                     const uint8_t* mask, const float* lse_n, float* dz_part, cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    k_dz_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)dy, mask, lse_n, dz_part)));
+    constexpr int RM = max_rows<kD, 2>();
+    FLARE_ROWS(RM, c.M, (long long)c.n_splits * c.B * c.H, k_dz_rows<T, kD, kR><<<dim3(c.n_splits, (c.M + 32 * kR - 1) / (32 * kR), c.B * c.H), kThreads, 0, st>>>(
+                            c, (const T*)q, (const T*)k, (const T*)dy, mask, lse_n, dz_part))
+    else k_dz_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)dy, mask, lse_n, dz_part)));
   return FLARE_OK;
 }
 
@@ -573,15 +1135,21 @@ int simt_dq_partial(const Ctx& c, int dtype, const void* q, const void* k, const
                     const uint8_t* mask, const float* z32, const float* dz32, const float* lse_m,
                     const float* lse_n, const float* delta_n, float* dq_part, cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    k_dq_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy,
-                                                         mask, z32, dz32, lse_m, lse_n, delta_n, dq_part)));
+    constexpr int RM = max_rows<kD, 4>();
+    FLARE_ROWS(RM, c.M, (long long)c.n_splits * c.B * c.H, k_dq_rows<T, kD, kR><<<dim3(c.n_splits, (c.M + 32 * kR - 1) / (32 * kR), c.B * c.H), kThreads, 0, st>>>(
+                            c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy, mask, z32, dz32, lse_m, lse_n, delta_n, dq_part))
+    else k_dq_partial<T, kD><<<lat_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy,
+                                                              mask, z32, dz32, lse_m, lse_n, delta_n, dq_part)));
   return FLARE_OK;
 }
 
 int simt_scatter(const Ctx& c, int dtype, const void* q, const void* k, const float* z32,
                  const uint8_t* mask, void* y, float* lse_n, cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    k_scatter<T, kD><<<tok_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, z32, mask, (T*)y, lse_n)));
+    constexpr int RM = max_rows<kD, 2>();
+    FLARE_ROWS(RM, c.N, (long long)c.B * c.H, k_scatter_rows<T, kD, kR><<<dim3((c.N + 32 * kR - 1) / (32 * kR), c.H, c.B), kThreads, 0, st>>>(
+                            c, (const T*)q, (const T*)k, z32, mask, (T*)y, lse_n))
+    else k_scatter<T, kD><<<tok_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, z32, mask, (T*)y, lse_n)));
   return FLARE_OK;
 }
 
@@ -590,17 +1158,26 @@ int simt_bwd_tokens(const Ctx& c, int dtype, const void* q, const void* k, const
                     const float* lse_m, const float* lse_n, void* dk, void* dv, float* delta_n,
                     cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    k_bwd_tokens<T, kD><<<tok_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy,
-                                                         (const T*)y, mask, z32, dz32, lse_m, lse_n,
-                                                         (T*)dk, (T*)dv, delta_n)));
+    constexpr int RM = max_rows<kD, 5>();
+    FLARE_ROWS(RM, c.N, (long long)c.B * c.H, k_bwd_tokens_rows<T, kD, kR><<<dim3((c.N + 32 * kR - 1) / (32 * kR), c.H, c.B), kThreads, 0, st>>>(
+                            c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy, (const T*)y, mask, z32, dz32, lse_m, lse_n,
+                            (T*)dk, (T*)dv, delta_n))
+    else k_bwd_tokens<T, kD><<<tok_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy,
+                                                              (const T*)y, mask, z32, dz32, lse_m, lse_n,
+                                                              (T*)dk, (T*)dv, delta_n)));
   return FLARE_OK;
 }
 
+template <typename Parts>
+static auto pick_combine(int D, int n_parts) -> decltype(&k_combine<4, 16, Parts>) {
+  if (D > 32) return &k_combine<4, 16, Parts>;
+  return n_parts <= 4 ? &k_combine<1, 4, Parts> : &k_combine<1, 16, Parts>;
+}
 int launch_combine(const float* rec, int n_parts, long long rows, int D, int dtype, float* z32,
                    void* z_out, float* lse_m, float* rec_out, cudaStream_t st) {
   const int rpb = kThreads / 32;
-  launch_dep(k_combine<PartsStrided>, dim3((unsigned)((rows + rpb - 1) / rpb)), dim3(kThreads), 0, st, PartsStrided{rec, rows * (D + 2)},
-             n_parts, rows, D, dtype, z32, z_out, lse_m, rec_out);
+  launch_dep(pick_combine<PartsStrided>(D, n_parts), dim3((unsigned)((rows + rpb - 1) / rpb)), dim3(kThreads), 0, st,
+             PartsStrided{rec, rows * (D + 2)}, n_parts, rows, D, dtype, z32, z_out, lse_m, rec_out);
   return FLARE_OK;
 }
 
@@ -614,8 +1191,8 @@ int launch_reduce_sum(const float* parts, int n_parts, long long n, float* out, 
 int launch_combine_ptrs(const float* const* recs, int n_parts, long long rows, int D, int dtype, float* z32,
                         void* z_out, float* lse_m, float* rec_out, cudaStream_t st) {
   const int rpb = kThreads / 32;
-  launch_dep(k_combine<PartsPtrs>, dim3((unsigned)((rows + rpb - 1) / rpb)), dim3(kThreads), 0, st, PartsPtrs{recs}, n_parts, rows, D,
-             dtype, z32, z_out, lse_m, rec_out);
+  launch_dep(pick_combine<PartsPtrs>(D, n_parts), dim3((unsigned)((rows + rpb - 1) / rpb)), dim3(kThreads), 0, st, PartsPtrs{recs},
+             n_parts, rows, D, dtype, z32, z_out, lse_m, rec_out);
   return FLARE_OK;
 }
 
