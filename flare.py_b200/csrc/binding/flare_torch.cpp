@@ -432,7 +432,7 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
     c10::cuda::CUDAGuard guard(k_.device());
     const Tensor q = latents(q_), k = tok(k_), v = tok(v_);
     FlareProblem p = problem(q, k, scale);
-    // the tensor-core shapes keep the chunk-start states for the backward (M (2 D + 8) bytes per 128 tokens and head);
+    // the tensor-core shapes keep the chunk-start states for the backward (M (4 D + 8) bytes per 128 tokens and head);
     // the others rebuild them there
     const size_t bytes = flare_causal_train_bytes(&p);
     Tensor y, saved;

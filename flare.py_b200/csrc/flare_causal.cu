@@ -55,11 +55,13 @@ constexpr int kScanRows = 2;      // rows per warp, walked side by side
 // the memory bandwidth.
 // COMPACT (behind the tensor-core record pass): the records are pacc[c][row][D] in 16 bits (what the tensor-core walk
 // multiplies with anyway) and pml[c][row] = (m, l), scanned in place like the fp32 ones: half the bytes in every
-// pass, and rows the walk can fetch in 16-byte pieces.  The sums themselves stay in fp32 registers.
-template <int D, bool COMPACT>
+// pass, and rows the walk can fetch in 16-byte pieces.  The sums themselves stay in fp32 registers.  LO: plo holds
+// the remainders of pacc (records and prefixes alike), for a backward pass.
+template <int D, bool COMPACT, bool LO>
 __global__ void __launch_bounds__(kScanThreads, D == 128 ? 5 : 8)
 k_causal_scan(float* __restrict__ rec, int n_chunks, long long rows, const float* __restrict__ state_in,
-              float* __restrict__ state_out, __nv_bfloat16* __restrict__ pacc, float2* __restrict__ pml) {
+              float* __restrict__ state_out, __nv_bfloat16* __restrict__ pacc, __nv_bfloat16* __restrict__ plo,
+              float2* __restrict__ pml) {
   grid_dep_sync();
   constexpr int W = D + 2;
   constexpr int VEC = D >= 64 ? 2 : 1;             // floats per access
@@ -109,8 +111,13 @@ k_causal_scan(float* __restrict__ rec, int n_chunks, long long rows, const float
         if constexpr (VEC == 2) {
           const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(pr + 64 * k + col));
           ab[q][u][k][0] = t.x; ab[q][u][k][1] = t.y;
+          if constexpr (LO) {
+            const float2 s = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(plo + i * D + 64 * k + col));
+            ab[q][u][k][0] += s.x; ab[q][u][k][1] += s.y;
+          }
         } else {
           ab[q][u][k][0] = lane_on ? __bfloat162float(pr[col]) : 0.f;
+          if (LO && lane_on) ab[q][u][k][0] += __bfloat162float(plo[i * D + col]);
         }
       }
     } else {
@@ -171,9 +178,19 @@ k_causal_scan(float* __restrict__ rec, int n_chunks, long long rows, const float
               __nv_bfloat16* pr = pacc + ((long long)c * rows + rw_[q]) * D;
 #pragma unroll
               for (int i = 0; i < NLD; ++i) {
-                if constexpr (VEC == 2)
-                  *reinterpret_cast<__nv_bfloat162*>(pr + 64 * i + col) = __floats2bfloat162_rn(acc[q][i][0], acc[q][i][1]);
-                else if (lane_on) pr[col] = __float2bfloat16_rn(acc[q][i][0]);
+                if constexpr (VEC == 2) {
+                  const __nv_bfloat162 hi = __floats2bfloat162_rn(acc[q][i][0], acc[q][i][1]);
+                  *reinterpret_cast<__nv_bfloat162*>(pr + 64 * i + col) = hi;
+                  if constexpr (LO) {
+                    const float2 f = __bfloat1622float2(hi);
+                    *reinterpret_cast<__nv_bfloat162*>(plo + ((long long)c * rows + rw_[q]) * D + 64 * i + col) =
+                        __floats2bfloat162_rn(acc[q][i][0] - f.x, acc[q][i][1] - f.y);
+                  }
+                } else if (lane_on) {
+                  const __nv_bfloat16 hi = __float2bfloat16_rn(acc[q][i][0]);
+                  pr[col] = hi;
+                  if constexpr (LO) plo[((long long)c * rows + rw_[q]) * D + col] = __float2bfloat16_rn(acc[q][i][0] - __bfloat162float(hi));
+                }
               }
               if (lane == 0) pml[(long long)c * rows + rw_[q]] = make_float2(m[q], l[q]);
             } else {
@@ -208,22 +225,23 @@ k_causal_scan(float* __restrict__ rec, int n_chunks, long long rows, const float
 }
 
 void launch_scan(bool dependent, float* rec, int n_chunks, long long rows, int D, const float* state_in, float* state_out,
-                 __nv_bfloat16* pacc, float2* pml, cudaStream_t st) {
+                 __nv_bfloat16* pacc, __nv_bfloat16* plo, float2* pml, cudaStream_t st) {
   const int rpb = kScanThreads / 32 * kScanRows;
   const dim3 grid((unsigned)((rows + rpb - 1) / rpb)), block(kScanThreads);
   auto go = [&](auto kernel) {
-    if (dependent) launch_dep(kernel, grid, block, 0, st, rec, n_chunks, rows, state_in, state_out, pacc, pml);
-    else kernel<<<grid, block, 0, st>>>(rec, n_chunks, rows, state_in, state_out, pacc, pml);
+    if (dependent) launch_dep(kernel, grid, block, 0, st, rec, n_chunks, rows, state_in, state_out, pacc, plo, pml);
+    else kernel<<<grid, block, 0, st>>>(rec, n_chunks, rows, state_in, state_out, pacc, plo, pml);
   };
   if (pacc) {                                      // behind the tensor-core record pass: D is 32 or 64
-    if (D == 32) go(k_causal_scan<32, true>); else go(k_causal_scan<64, true>);
+    if (plo) { if (D == 32) go(k_causal_scan<32, true, true>); else go(k_causal_scan<64, true, true>); }
+    else { if (D == 32) go(k_causal_scan<32, true, false>); else go(k_causal_scan<64, true, false>); }
     return;
   }
   switch (D) {                                     // fill_args admits exactly these
-    case 16: go(k_causal_scan<16, false>); break;
-    case 32: go(k_causal_scan<32, false>); break;
-    case 64: go(k_causal_scan<64, false>); break;
-    default: go(k_causal_scan<128, false>); break;
+    case 16: go(k_causal_scan<16, false, false>); break;
+    case 32: go(k_causal_scan<32, false, false>); break;
+    case 64: go(k_causal_scan<64, false, false>); break;
+    default: go(k_causal_scan<128, false, false>); break;
   }
 }
 
@@ -527,27 +545,27 @@ namespace flare {
 // pass 2 for the backward (flare_causal_bwd.cu), which needs the same chunk-start records
 int launch_causal_scan(float* rec, int n_chunks, long long rows, int D, const float* state_in, float* state_out,
                        cudaStream_t st) {
-  launch_scan(false, rec, n_chunks, rows, D, state_in, state_out, nullptr, nullptr, st);
+  launch_scan(false, rec, n_chunks, rows, D, state_in, state_out, nullptr, nullptr, nullptr, st);
   const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return refuse(FLARE_ECUDA, "causal scan: %s", cudaGetErrorString(e));
   return FLARE_OK;
 }
 
-int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc, float2* pml,
-                     const float* state_in, float* state_out, int chunks, cudaStream_t st) {
-  const int rc = causal_tc_record(p, q, k, v, pacc, pml, chunks, st);
+int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc, __nv_bfloat16* plo,
+                     float2* pml, const float* state_in, float* state_out, int chunks, cudaStream_t st) {
+  const int rc = causal_tc_record(p, q, k, v, pacc, plo, pml, chunks, st);
   if (rc != FLARE_OK) return refuse(rc, "causal: tensor-core record pass could not be launched");
-  launch_scan(true, nullptr, chunks, (long long)p->B * p->H * p->M, p->D, state_in, state_out, pacc, pml, st);
+  launch_scan(true, nullptr, chunks, (long long)p->B * p->H * p->M, p->D, state_in, state_out, pacc, plo, pml, st);
   return FLARE_OK;
 }
 
 int causal_tc_prefill(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, __nv_bfloat16* pacc,
-                      float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st) {
+                      __nv_bfloat16* plo, float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st) {
   CausalArgs a;
   int rc = fill_args(p, &a);
   if (rc != FLARE_OK) return rc;
   const int chunks = (p->N + kChunk - 1) / kChunk;
-  rc = causal_tc_prefix(p, q, k, v, pacc, pml, state_in, state_out, chunks, st);
+  rc = causal_tc_prefix(p, q, k, v, pacc, plo, pml, state_in, state_out, chunks, st);
   if (rc != FLARE_OK) return rc;
   // the tensor-core walk flags the chunks whose scores span too many octaves for its fixed reference
   // maximum; the fp32 walk, launched behind it, redoes exactly those (every other CTA returns at once)
@@ -591,7 +609,7 @@ int flare_causal_prefill(const FlareProblem* p, const void* q, const void* k, co
     wsb += ((size_t)chunks * p->B * p->H * sizeof(int) + 15) & ~size_t(15);
     float2* pml = reinterpret_cast<float2*>(wsb);
     wsb += (size_t)chunks * rows * sizeof(float2);
-    return flare::causal_tc_prefill(p, q, k, v, y, reinterpret_cast<__nv_bfloat16*>(wsb), pml, redo, state_in, state_out, st);
+    return flare::causal_tc_prefill(p, q, k, v, y, reinterpret_cast<__nv_bfloat16*>(wsb), nullptr, pml, redo, state_in, state_out, st);
   }
   // pass 1: one record per 128-token chunk
   FlareProblem pp = *p;
@@ -599,7 +617,7 @@ int flare_causal_prefill(const FlareProblem* p, const void* q, const void* k, co
   rc = flare_gather_partial(&pp, q, k, v, nullptr, workspace, st);
   if (rc != FLARE_OK) return rc;
   // pass 2: exclusive prefix along the chunk axis
-  launch_scan(true, workspace, chunks, rows, p->D, state_in, state_out, nullptr, nullptr, st);
+  launch_scan(true, workspace, chunks, rows, p->D, state_in, state_out, nullptr, nullptr, nullptr, st);
   // pass 3: the tokens of every chunk
   a.q = q; a.k = k; a.v = v; a.y = y;
   a.prefix = workspace; a.state = nullptr; a.tokens_per_cta = kChunk;

@@ -61,7 +61,8 @@ struct CausalBwdArgs {
   float* sub;                  // [B*H][4][M][D+2]: records before sub-chunks 1..3 of the current chunk; slot 3 (redo): the chunk's own
   // behind the tensor-core backward: only the (b, h) whose flag is set, their prefixes in the 16-bit form
   const int* redo;
-  const __nv_bfloat16* pacc;   // [n_chunks][B][H][M][D]
+  const __nv_bfloat16* pacc;   // [n_chunks][B][H][M][D], with the remainders in plo
+  const __nv_bfloat16* plo;
   const float2* pml;           // [n_chunks][B][H][M]
   int units;                   // redo: dq holds this many partials [B*H][D/4][128][4], unscaled: this kernel's in the first, zeros in the others
 };
@@ -181,7 +182,7 @@ k_causal_bwd(CausalBwdArgs a) {
     const float* pre = a.prefix + prow * W;
     if (a.redo) {
       float* own = subst + 3LL * M * W;
-      for (int i = tid; i < MD; i += kThreads) own[(i / D) * W + i % D] = to_f32(a.pacc[prow * D + i]);
+      for (int i = tid; i < MD; i += kThreads) own[(i / D) * W + i % D] = to_f32(a.pacc[prow * D + i]) + to_f32(a.plo[prow * D + i]);
       for (int m = tid; m < M; m += kThreads) { own[m * W + D] = a.pml[prow + m].x; own[m * W + D + 1] = a.pml[prow + m].y; }
       pre = own;
       __syncthreads();
@@ -414,10 +415,12 @@ int check_args(const FlareProblem* p, const void* q, const void* k, const void* 
   return FLARE_OK;
 }
 
-// The compact prefixes inside a caller's buffer: redo flags of the forward walk | (m, l) pairs | acc rows.
+// The compact prefixes inside a caller's buffer: redo flags of the forward walk | (m, l) pairs | acc rows | their
+// remainders.
 struct Prefix {
   float2* pml;
   __nv_bfloat16* pacc;
+  __nv_bfloat16* plo;
   int* redo;
   Prefix(const FlareProblem* p, void* saved) {
     const size_t chunks = ((size_t)p->N + kChunk - 1) / kChunk, BH = (size_t)p->B * p->H;
@@ -425,11 +428,12 @@ struct Prefix {
     redo = reinterpret_cast<int*>(w);
     w += (chunks * BH * sizeof(int) + 15) & ~size_t(15);
     pml = reinterpret_cast<float2*>(w);
-    pacc = reinterpret_cast<__nv_bfloat16*>(w + chunks * BH * p->M * sizeof(float2));
+    pacc = reinterpret_cast<__nv_bfloat16*>(w + ((chunks * BH * p->M * sizeof(float2) + 15) & ~size_t(15)));
+    plo = pacc + chunks * BH * p->M * p->D;
   }
   static size_t bytes(const FlareProblem* p) {
     const size_t chunks = ((size_t)p->N + kChunk - 1) / kChunk, BH = (size_t)p->B * p->H;
-    return ((chunks * BH * sizeof(int) + 15) & ~size_t(15)) + chunks * BH * p->M * (sizeof(float2) + 2 * (size_t)p->D) + 32;
+    return ((chunks * BH * sizeof(int) + 15) & ~size_t(15)) + chunks * BH * p->M * (sizeof(float2) + 4 * (size_t)p->D) + 48;
   }
 };
 
@@ -446,11 +450,11 @@ int launch_causal_scan(float* rec, int n_chunks, long long rows, int D, const fl
                        cudaStream_t st);
 
 int causal_bwd_redo(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
-                    const __nv_bfloat16* pacc, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
+                    const __nv_bfloat16* pacc, const __nv_bfloat16* plo, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
                     void* dv, float* sub, cudaStream_t st) {
   CausalBwdArgs a = fill(p, q, k, v, dy, dk, dv);
   a.dq = dq_part; a.units = units; a.sub = sub;
-  a.redo = redo; a.pacc = pacc; a.pml = pml;
+  a.redo = redo; a.pacc = pacc; a.plo = plo; a.pml = pml;
   return launch<__nv_bfloat16>(a, st);
 }
 }  // namespace flare
@@ -482,9 +486,9 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
   if (causal_bwd_tc_supported(p, q, k, v, dy, dk, dv)) {
     // one chunk per CTA on the tensor cores, behind the forward's record and scan passes
     const Prefix pre(p, workspace);
-    int rc = causal_tc_prefix(p, q, k, v, pre.pacc, pre.pml, nullptr, nullptr, chunks, st);
+    int rc = causal_tc_prefix(p, q, k, v, pre.pacc, pre.plo, pre.pml, nullptr, nullptr, chunks, st);
     if (rc == FLARE_OK)
-      rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.pml, dq32, false, dk, dv,
+      rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.plo, pre.pml, dq32, false, dk, dv,
                          reinterpret_cast<char*>(workspace) + Prefix::bytes(p), st);
     return rc == FLARE_OK ? rc : refuse(rc, "causal_bwd: tensor-core pass could not be launched");
   }
@@ -516,7 +520,7 @@ int flare_causal_train_fwd(const FlareProblem* p, const void* q, const void* k, 
   if (!p || !q || !k || !v || !y || !saved) return refuse(FLARE_EINVAL, "causal_train_fwd: null pointer");
   if (!causal_tc_walk_supported(p, q, k, v, y)) return refuse(FLARE_EUNSUPPORTED, "causal_train_fwd: bf16, M <= 128, D in {32,64}, 16-byte aligned rows only");
   const Prefix pre(p, saved);
-  return causal_tc_prefill(p, q, k, v, y, pre.pacc, pre.pml, pre.redo, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+  return causal_tc_prefill(p, q, k, v, y, pre.pacc, pre.plo, pre.pml, pre.redo, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int flare_causal_train_bwd(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const void* saved,
@@ -527,7 +531,7 @@ int flare_causal_train_bwd(const FlareProblem* p, const void* q, const void* k, 
   if (!causal_bwd_tc_supported(p, q, k, v, dy, dk, dv))
     return refuse(FLARE_EUNSUPPORTED, "causal_train_bwd: bf16, M <= 128, D in {32,64}, 16-byte aligned rows only");
   const Prefix pre(p, const_cast<void*>(saved));
-  const int rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.pml, dq32, p->q_stride[0] == 0, dk, dv, workspace, static_cast<cudaStream_t>(stream));
+  const int rc = causal_bwd_tc(p, q, k, v, dy, pre.pacc, pre.plo, pre.pml, dq32, p->q_stride[0] == 0, dk, dv, workspace, static_cast<cudaStream_t>(stream));
   return rc == FLARE_OK ? rc : refuse(rc, "causal_train_bwd: tensor-core pass could not be launched");
 }
 

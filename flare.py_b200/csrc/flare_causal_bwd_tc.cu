@@ -20,17 +20,20 @@
 // middle of a chunk: everything up to c and Gg is independent of it, and a chunk publishes its own state as soon as it
 // has read its predecessor's.  Before this kernel one CTA per (b, h) walked its chunks alone in fp32 FMA loops.
 //
-// Operands.  Every 128 x 128 operand is written where the next product reads it: rows of E, G, dS both packed in tensor
+// Operands.  Every 128 x 128 operand is written where the next product reads it: rows of E, G, dS packed in tensor
 // memory (A operand, contraction over the tokens) and as 64-token column blocks in shared memory (MN-major operand,
 // contraction over the latents); X once, masked to t >= n, serves as the MN-major operand of C and the K-major operand
-// of de.  X, dS, W and G (in de) are carried as two bf16 terms (value and remainder), so that the contractions see
-// about 16 bits of them: those are the roundings that would dominate the error of dq, dk, dv (each 1.2e-3 to 1.6e-3
-// relative with one term at M = 128, D = 64, N = 2048; 2.8e-3 in all).
+// of de.  All of them, and a acc0, Rin and W, are carried as two bf16 terms (value and remainder), so that the
+// contractions see about 16 bits and the error of dq, dk, dv is that of rounding the results: with one term of E, G in
+// W and Gg, a acc0 and Rin they were 2.23e-3, 2.08e-3, 1.74e-3 off (B = 1, H = 8, N = 512, M = 128, D = 64; rounding
+// alone is 1.67e-3), now 1.72e-3, 1.71e-3, 1.68e-3, as in the fp32 kernel.  Shared memory has room for one pair of remainders at a time: first those
+// of E and G, for W; then X, which waits in tensor memory until W is complete; then dS.  The second term of E^T Rin comes
+// last, over E.
 //
 // Tensor memory (512 columns):   0 S | E, G packed | G remainder over E | dS, dS remainder
 //                              128 S^T | W^T | W packed in place
 //                              256 X | C | de | dk
-//                              384 dq of the unit      448 Gg | dv
+//                              384 E remainder | dq of the unit      448 a acc0 remainder | Gg | dv
 //
 // Range: E, l and G are relative to the chunk's final maximum, as in the forward walk, with the same bounds (64
 // octaves of climb, 50 between the latents' maxima and the first token's column maximum).  A (b, h) with a chunk
@@ -56,7 +59,8 @@ struct CausalBwdTcArgs {
   int chunks;
   float scale, scale_log2;
   int q_batched;
-  const __nv_bfloat16* pacc;                       // prefix of every chunk as the scan left it
+  const __nv_bfloat16* pacc;                       // prefix of every chunk as the scan left it, in two terms
+  const __nv_bfloat16* plo;
   const float2* pml;
   float4* dq_part;                                 // [chunks][B*H][D/4][128]: four columns of a latent's dq, not yet scaled
   float4* carry;                                   // [B*H][D/4][128]: R of the chunk handed on
@@ -161,12 +165,14 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 128);
   uint64_t* bar_ld = bars;                         // Q, K, V, g landed
   uint64_t* bar_s = bars + 1;                      // S, S^T, X complete
-  uint64_t* bar_c = bars + 2;                      // C and Gg complete
+  uint64_t* bar_c = bars + 2;                      // C complete
   uint64_t* bar_w = bars + 3;                      // W^T complete
   uint64_t* bar_de = bars + 4;                     // de complete
   uint64_t* bar_out = bars + 5;                    // dv, dk, dq complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
-  int* abort_flag = reinterpret_cast<int*>(bars + 7);
+  uint64_t* bar_g = bars + 6;                      // Gg complete
+  uint64_t* bar_e = bars + 7;                      // E in shared memory has been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  int* abort_flag = reinterpret_cast<int*>(bars + 9);
   int* sNext = abort_flag + 1;                     // the chunk after this one
   int* sReady = abort_flag + 2;                    // the predecessor's state was out when E and G were
 
@@ -177,7 +183,7 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const float sl = a.scale_log2;
 
   if (tid == 0) {
-    for (int i = 0; i < 6; ++i) mbar_init(bars + i, 1);
+    for (int i = 0; i < 8; ++i) mbar_init(bars + i, 1);
     abort_flag[0] = 0;
     *sNext = atomicAdd(a.sync, 1);
     fence_barrier_init();
@@ -189,7 +195,7 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t row = tmem + ((uint32_t)(rb * 32) << 16);
-  constexpr uint32_t cS = 0, cEh = 0, cGh = 64, cGl = 0, cDSh = 0, cDSl = 64, cT = 128, cX = 256, cDQ = 384, cDV = 448;
+  constexpr uint32_t cS = 0, cEh = 0, cGh = 64, cGl = 0, cDSh = 0, cDSl = 64, cT = 128, cX = 256, cEl = 384, cDQ = 384, cDV = 448, cAl = cDV;
 
   const uint32_t id_s = idesc_f16(128, 128, 1, 1, 0, 0);            // A, B K-major, N = 128
   const uint32_t id_mn = idesc_f16(128, 128, 1, 1, 1, 1);           // A, B MN-major, N = 128
@@ -197,7 +203,7 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t id_td = idesc_f16(128, D, 1, 1, 0, 1);             // the same, N = D
   const uint32_t id_md = idesc_f16(128, D, 1, 1, 1, 1);             // A, B MN-major, N = D
   const uint64_t dQ = smem_desc<ROWB>(smem_u32(sQ)), dK = smem_desc<ROWB>(smem_u32(sK)), dV = smem_desc<ROWB>(smem_u32(sV)),
-                 dg = smem_desc<ROWB>(smem_u32(sg)), dAR = smem_desc<ROWB>(smem_u32(sAR));
+                 dg = smem_desc<ROWB>(smem_u32(sg)), dAR = smem_desc<ROWB>(smem_u32(sAR)), dRl = smem_desc<ROWB>(smem_u32(sG));
   const uint64_t dE = smem_desc_mn128(smem_u32(sE), kHalf, 1024), dG = smem_desc_mn128(smem_u32(sG), kHalf, 1024),
                  dXh = smem_desc_mn128(smem_u32(sXh), kHalf, 1024), dXl = smem_desc_mn128(smem_u32(sXl), kHalf, 1024);
 
@@ -264,11 +270,17 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       __syncwarp();
     }
+    uint4 al[NP];                                  // remainders of this thread's piece of acc0
+    {
+      const uint4* src = reinterpret_cast<const uint4*>(a.plo + ((((long long)c * a.B * a.H + bh) * M) + min(r, M - 1)) * D) + w * NP;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) al[i] = __ldcs(src + i);
+    }
     const float m0l = ml0.x * kLog2e;              // the record keeps m in natural-log units
     const float l0 = ml0.y;
     mbar_wait_hot(bar_s, ph, a.status, abort_flag);
     tc_fence_after();
-    // ---- token r over 32 latents: maximum and sum.  X: mask and pack.  latent r over its 32 tokens: maximum ----
+    // ---- token r over 32 latents: maximum and sum.  latent r over its 32 tokens: maximum ----
     uint32_t v[32], hi[16], lo[16];
     tmem_ld32(row + cT + 32 * w, v);
     tmem_wait_ld_on(v);
@@ -290,11 +302,6 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       sPart[w * 128 + r] = make_float2(mx, su);
     }
-    tmem_ld32(row + cX + 32 * w, v);
-    tmem_wait_ld_on(v);
-    split_upper(v, w, rb, lane, hi, lo);
-    put_row(sXh, r, w, hi);
-    put_row(sXl, r, w, lo);
     tmem_ld32(row + cS + 32 * w, v);
     tmem_wait_ld_on(v);
     const float first = fmaxf(m0l, __uint_as_float(v[0]) * sl);     // w == 0: the running maximum after the chunk's first token
@@ -334,21 +341,20 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (w == 0 && live && (mu - first > 64.f || fabsf(mu - c0) > 50.f)) a.redo[bh] = 1;
     const float um = live ? ex2(fminf(fmaxf(mu - c0, -60.f), 60.f)) : 0.f;
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {                 // a acc0 in place
+    for (int i = 0; i < NP; ++i) {                 // a acc0 in place, its remainder where Gg will be
       uint4* at = reinterpret_cast<uint4*>(sAR + swz_off<ROWB>(r, w * NP + i));
-      uint4 o = make_uint4(0, 0, 0, 0);
+      uint32_t ow[4] = {0u, 0u, 0u, 0u}, lw[4] = {0u, 0u, 0u, 0u};
       if (live) {
         const uint4 s4 = *at;
-        const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
-        uint32_t ow[4];
+        const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w}, tw[4] = {al[i].x, al[i].y, al[i].z, al[i].w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const float2 f = Op16<__nv_bfloat16>::unpack(sw[u]);
-          ow[u] = pack_bf16(f.x * aa, f.y * aa);
+          const float2 f = Op16<__nv_bfloat16>::unpack(sw[u]), g = Op16<__nv_bfloat16>::unpack(tw[u]);
+          split2((f.x + g.x) * aa, (f.y + g.y) * aa, ow[u], lw[u]);
         }
-        o = make_uint4(ow[0], ow[1], ow[2], ow[3]);
       }
-      *at = o;
+      *at = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+      tmem_st4(row + cAl + 4 * (w * NP + i), lw);
     }
     // ---- E ----
     float e[32];
@@ -372,6 +378,11 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (warp == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncthreads();
     tmem_st16(row + cEh + 16 * w, hi);             // every row of S has been read
+#pragma unroll
+    for (int j = 0; j < 16; ++j)                   // what the 16 bits of E left over, for C and W
+      hi[j] = pack_bf16(e[2 * j] - __uint_as_float(hi[j] << 16), e[2 * j + 1] - __uint_as_float(hi[j] & 0xffff0000u));
+    tmem_st16(row + cEl + 16 * w, hi);
+    put_row(sXh, r, w, hi);                        // until W is complete; then X
     // ---- l, A, G ----
     const float4* wt4 = reinterpret_cast<const float4*>(sWt + 32 * w);
     float il[32];                                  // 1 / l
@@ -392,11 +403,12 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           il[j] = l > 0.f ? rcp(l) : 0.f;          // l = 0: a latent row past M, or a chunk that is flagged and redone
           g[u] = e[j] * (um * ws[u]) * il[j];
         }
-        lo[2 * q] = pack_bf16(g[0], g[1]);
-        lo[2 * q + 1] = pack_bf16(g[2], g[3]);
+        split2(g[0], g[1], lo[2 * q], hi[2 * q]);
+        split2(g[2], g[3], lo[2 * q + 1], hi[2 * q + 1]);
       }
       tmem_st16(row + cGh + 16 * w, lo);
       put_row(sG, r, w, lo);
+      put_row(sXl, r, w, hi);
     }
     if (tid == kRowT - 1) *sReady = last || ld_acquire(a.sync + 1 + (c + 1) * BH + bh) != 0;
     tmem_wait_st();
@@ -407,26 +419,46 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(tmem + cT, dE + 128 * kk, dG + 128 * kk, id_mn, kk > 0);       // over the latents
-        mma_commit(bar_w);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cX, dAR + 2 * kk, dg + 2 * kk, id_s, kk > 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {           // contraction over the tokens n, 16 per product
-          mma_ts(tmem + cX, tmem + cEh + 8 * kk, dXh + 128 * kk, id_tm, true);
-          mma_ts(tmem + cX, tmem + cEh + 8 * kk, dXl + 128 * kk, id_tm, true);
+        for (int kk = 0; kk < 8; ++kk) {           // over the latents
+          mma_ss(tmem + cT, dE + 128 * kk, dG + 128 * kk, id_mn, kk > 0);
+          mma_ss(tmem + cT, dXh + 128 * kk, dG + 128 * kk, id_mn, true);
+          mma_ss(tmem + cT, dE + 128 * kk, dXl + 128 * kk, id_mn, true);
         }
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ts(tmem + cDV, tmem + cGh + 8 * kk, dg + (uint64_t)(kk * ROWB), id_td, kk > 0);
-        mma_commit(bar_c);
+        mma_commit(bar_w);
       }
       __syncwarp();
     }
     const bool ready = *reinterpret_cast<volatile int*>(sReady) != 0;
 
-    // ---- W^T of token r, masked to t >= r, packed in place, while C is formed ----
+    // ---- X of token r, masked to t >= r, packed over the remainders; then W^T likewise, in place, while C is formed ----
+    tmem_ld32(row + cX + 32 * w, v);
+    tmem_wait_ld_on(v);
+    split_upper(v, w, rb, lane, hi, lo);
     mbar_wait_hot(bar_w, ph, a.status, abort_flag);
+    put_row(sXh, r, w, hi);
+    put_row(sXl, r, w, lo);
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
     tc_fence_after();
+    if (warp == 0) {
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) mma_ts(tmem + cX, tmem + cAl + 8 * kk, dg + 2 * kk, id_s, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cX, dAR + 2 * kk, dg + 2 * kk, id_s, true);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {           // contraction over the tokens n, 16 per product
+          mma_ts(tmem + cX, tmem + cEh + 8 * kk, dXh + 128 * kk, id_tm, true);
+          mma_ts(tmem + cX, tmem + cEh + 8 * kk, dXl + 128 * kk, id_tm, true);
+          mma_ts(tmem + cX, tmem + cEl + 8 * kk, dXh + 128 * kk, id_tm, true);
+        }
+        mma_commit(bar_c);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) mma_ts(tmem + cDV, tmem + cGh + 8 * kk, dg + (uint64_t)(kk * ROWB), id_td, kk > 0);
+      }
+      __syncwarp();
+    }
     tmem_ld32(row + cT + 32 * w, v);
     tmem_wait_ld_on(v);
     split_upper(v, w, rb, lane, hi, lo);
@@ -500,7 +532,18 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     }
+    tmem_wait_st();
+    tc_fence_before();
     __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) mma_ts(tmem + cDV, tmem + cGl + 8 * kk, dg + (uint64_t)(kk * ROWB), id_td, true);
+        mma_commit(bar_g);
+      }
+      __syncwarp();
+    }
     if (!ready) take();
     float after, gc_all;                           // sums of G c: the quarters behind this one, the chunk
     {
@@ -512,22 +555,26 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const float wf = last ? 0.f : ex2(mu - rnu.y);
     const float rin = wf * rnu.x;
     {
-      uint32_t gg[DQ], rp[DQ / 2];
+      uint32_t gg[DQ], rp[DQ / 2], rl[DQ / 2];
+      mbar_wait_hot(bar_g, ph, a.status, abort_flag);
+      tc_fence_after();
       if constexpr (DQ == 16) tmem_ld16(row + cDV + DQ * w, gg);
       else tmem_ld8(row + cDV + DQ * w, gg);
       tmem_wait_ld();
 #pragma unroll
       for (int p = 0; p < DQ / 4; ++p) {
         const float4 in4 = make_float4(st[p].x * wf, st[p].y * wf, st[p].z * wf, st[p].w * wf);
-        rp[2 * p] = pack_bf16(in4.x, in4.y);
-        rp[2 * p + 1] = pack_bf16(in4.z, in4.w);
+        split2(in4.x, in4.y, rp[2 * p], rl[2 * p]);
+        split2(in4.z, in4.w, rp[2 * p + 1], rl[2 * p + 1]);
         if (c > 0)
           cp[p * 128] = make_float4(in4.x + __uint_as_float(gg[4 * p]), in4.y + __uint_as_float(gg[4 * p + 1]),
                                     in4.z + __uint_as_float(gg[4 * p + 2]), in4.w + __uint_as_float(gg[4 * p + 3]));
       }
 #pragma unroll
-      for (int i = 0; i < NP; ++i)                 // Rin over a acc0: C is complete
+      for (int i = 0; i < NP; ++i) {               // Rin over a acc0, its remainder over G: C and W are complete
         *reinterpret_cast<uint4*>(sAR + swz_off<ROWB>(r, w * NP + i)) = make_uint4(rp[4 * i], rp[4 * i + 1], rp[4 * i + 2], rp[4 * i + 3]);
+        *reinterpret_cast<uint4*>(sG + swz_off<ROWB>(r, w * NP + i)) = make_uint4(rl[4 * i], rl[4 * i + 1], rl[4 * i + 2], rl[4 * i + 3]);
+      }
       if (w == 0 && c > 0) cml[128 * (c & 1)] = make_float2(rin - gc_all, mu);
     }
     tmem_wait_st();
@@ -542,7 +589,10 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) mma_ss(tmem + cX, dAR + 2 * kk, dV + 2 * kk, id_s, kk > 0);
+        for (int kk = 0; kk < D / 16; ++kk) {
+          mma_ss(tmem + cX, dAR + 2 * kk, dV + 2 * kk, id_s, kk > 0);
+          mma_ss(tmem + cX, dRl + 2 * kk, dV + 2 * kk, id_s, true);
+        }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {           // contraction over the tokens t: X as a K-major operand
           const uint64_t kh = smem_desc<128>(smem_u32(sXh) + (kk >> 2) * kHalf) + 2 * (kk & 3);
@@ -553,7 +603,11 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         mma_commit(bar_de);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(tmem + cDV, dE + 128 * kk, dAR + (uint64_t)(kk * ROWB), id_md, kk > 0);
+        for (int kk = 0; kk < 8; ++kk) {
+          mma_ss(tmem + cDV, dE + 128 * kk, dAR + (uint64_t)(kk * ROWB), id_md, kk > 0);
+          mma_ss(tmem + cDV, dE + 128 * kk, dRl + (uint64_t)(kk * ROWB), id_md, true);
+        }
+        mma_commit(bar_e);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {           // W packed in place: 16 columns of values, 16 of remainders per quarter
           const uint32_t wp = tmem + cT + 32 * (kk >> 1) + 8 * (kk & 1);
@@ -587,6 +641,13 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tmem_st16(row + cDSl + 16 * w, lo);
     put_row(sXh, r, w, hi);                        // over X: de is complete
     put_row(sXl, r, w, lo);
+    mbar_wait_hot(bar_e, ph, a.status, abort_flag);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {                 // the remainder of E over E, for dv
+      uint32_t eh;
+      split2(e[2 * j], e[2 * j + 1], eh, lo[j]);
+    }
+    put_row(sE, r, w, lo);
     tmem_wait_st();
     fence_proxy_async();
     tc_fence_before();
@@ -596,6 +657,7 @@ k_causal_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
+          mma_ss(tmem + cDV, dE + 128 * kk, dAR + (uint64_t)(kk * ROWB), id_md, true);
           mma_ss(tmem + cX, dXh + 128 * kk, dQ + (uint64_t)(kk * ROWB), id_md, kk > 0);              // dk over de
           mma_ss(tmem + cX, dXl + 128 * kk, dQ + (uint64_t)(kk * ROWB), id_md, true);
           mma_ts(tmem + cDQ, tmem + cDSh + 8 * kk, dK + (uint64_t)(kk * ROWB), id_td, kk > 0);
@@ -732,7 +794,7 @@ bool causal_bwd_tc_supported(const FlareProblem* p, const void* q, const void* k
 size_t causal_bwd_tc_workspace(const FlareProblem* p) { return layout(p).total; }
 
 int causal_bwd_tc(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const __nv_bfloat16* pacc,
-                  const float2* pml, float* dq32, bool sum_batch, void* dk, void* dv, void* workspace, cudaStream_t st) {
+                  const __nv_bfloat16* plo, const float2* pml, float* dq32, bool sum_batch, void* dk, void* dv, void* workspace, cudaStream_t st) {
   const BwdLayout L = layout(p);
   char* ws = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   const int BH = p->B * p->H;
@@ -741,7 +803,7 @@ int causal_bwd_tc(const FlareProblem* p, const void* q, const void* k, const voi
   a.chunks = L.chunks;
   a.scale = p->scale; a.scale_log2 = p->scale * kLog2e;
   a.q_batched = p->q_stride[0] != 0;
-  a.pacc = pacc; a.pml = pml;
+  a.pacc = pacc; a.plo = plo; a.pml = pml;
   a.dq_part = reinterpret_cast<float4*>(ws + L.part);
   a.carry = reinterpret_cast<float4*>(ws + L.carry);
   a.carry_ml = reinterpret_cast<float2*>(ws + L.carry_ml);
@@ -751,7 +813,7 @@ int causal_bwd_tc(const FlareProblem* p, const void* q, const void* k, const voi
   if (cudaMemsetAsync(a.sync, 0, (1 + (size_t)L.chunks * BH + BH) * sizeof(int), st) != cudaSuccess) return FLARE_ECUDA;
   int rc = p->D == 32 ? launch_bwd<32>(p, q, k, v, dy, dk, dv, a, st) : launch_bwd<64>(p, q, k, v, dy, dk, dv, a, st);
   if (rc != FLARE_OK) return rc;
-  rc = causal_bwd_redo(p, q, k, v, dy, pacc, pml, a.redo, reinterpret_cast<float*>(a.dq_part), L.chunks, dk, dv, reinterpret_cast<float*>(ws + L.sub), st);
+  rc = causal_bwd_redo(p, q, k, v, dy, pacc, plo, pml, a.redo, reinterpret_cast<float*>(a.dq_part), L.chunks, dk, dv, reinterpret_cast<float*>(ws + L.sub), st);
   if (rc != FLARE_OK) return rc;
   const int heads = sum_batch ? p->H : BH, parts = L.chunks * (sum_batch ? p->B : 1);
   const dim3 grid((unsigned)((p->M + 31) / 32), (unsigned)(p->D / 4), (unsigned)heads);

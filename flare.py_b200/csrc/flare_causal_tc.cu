@@ -377,11 +377,12 @@ k_causal_tc_walk(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // m = rowmax, E = e^{S - m} packed to bf16 in place in tensor memory, acc = E V.  128 tensor-memory columns and
 // three operand tiles per CTA: four CTAs per SM.  acc leaves in 16 bits through shared memory as one contiguous block
 // (the scan adds the records up in fp32; the walk multiplies 16-bit operands anyway), (m, l) as one pair per latent.
-template <int D>
+// LO: also rlo, what the 16 bits left over of acc, in 16 bits more, for a backward pass.
+template <int D, bool LO>
 __global__ void __launch_bounds__(kThreadsW, 4)
 k_causal_tc_record(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, CausalTcArgs a, __nv_bfloat16* __restrict__ racc,
-                   float2* __restrict__ rml) {
+                   __nv_bfloat16* __restrict__ rlo, float2* __restrict__ rml) {
   grid_dep_sync();
   constexpr int ROWB = 2 * D;
   constexpr int kTile = 128 * ROWB;
@@ -489,6 +490,16 @@ k_causal_tc_record(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         o.z = pack_bf16(__uint_as_float(v[8 * q4 + 4]), __uint_as_float(v[8 * q4 + 5]));
         o.w = pack_bf16(__uint_as_float(v[8 * q4 + 6]), __uint_as_float(v[8 * q4 + 7]));
         *reinterpret_cast<uint4*>(sOut + swz_off<ROWB>(r, 4 * c + q4)) = o;
+        if constexpr (LO) {
+          const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+          uint32_t lw[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float2 f = Op16<__nv_bfloat16>::unpack(ow[u]);
+            lw[u] = pack_bf16(__uint_as_float(v[8 * q4 + 2 * u]) - f.x, __uint_as_float(v[8 * q4 + 2 * u + 1]) - f.y);
+          }
+          *reinterpret_cast<uint4*>(sOut + kTile + swz_off<ROWB>(r, 4 * c + q4)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        }
       }
     }
     if (r < M && !*reinterpret_cast<volatile int*>(abort_flag)) rml[prow + r] = make_float2(mx * kLn2, l);
@@ -499,6 +510,10 @@ k_causal_tc_record(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint4* dst = reinterpret_cast<uint4*>(racc + prow * D);
     constexpr int CPR = ROWB / 16;
     for (int i = tid; i < M * CPR; i += kThreadsW) dst[i] = *reinterpret_cast<const uint4*>(sOut + swz_off<ROWB>(i / CPR, i % CPR));
+    if constexpr (LO) {
+      uint4* dlo = reinterpret_cast<uint4*>(rlo + prow * D);
+      for (int i = tid; i < M * CPR; i += kThreadsW) dlo[i] = *reinterpret_cast<const uint4*>(sOut + kTile + swz_off<ROWB>(i / CPR, i % CPR));
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -550,15 +565,15 @@ int launch_walk_tc(const FlareProblem* p, const void* q, const void* k, const vo
 }
 
 template <int D>
-int launch_record_tc(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, float2* rml,
+int launch_record_tc(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, __nv_bfloat16* rlo, float2* rml,
                      int chunks, cudaStream_t st) {
   TcLaunch L;
   const int rc = fill_launch<D>(p, q, k, v, &L);
   if (rc != FLARE_OK) return rc;
   constexpr int smem = 3 * 128 * 2 * D + 256 + 1024;
-  if (tc_set_dyn_smem(reinterpret_cast<const void*>(&k_causal_tc_record<D>), smem) != FLARE_OK) return FLARE_ECUDA;
-  launch_dep(k_causal_tc_record<D>, dim3((unsigned)chunks, (unsigned)(p->B * p->H)), dim3(kThreadsW), smem, st, L.tmQ, L.tmK,
-             L.tmV, L.a, racc, rml);
+  const auto kernel = rlo ? &k_causal_tc_record<D, true> : &k_causal_tc_record<D, false>;
+  if (tc_set_dyn_smem(reinterpret_cast<const void*>(kernel), smem) != FLARE_OK) return FLARE_ECUDA;
+  launch_dep(kernel, dim3((unsigned)chunks, (unsigned)(p->B * p->H)), dim3(kThreadsW), smem, st, L.tmQ, L.tmK, L.tmV, L.a, racc, rlo, rml);
   return FLARE_OK;
 }
 
@@ -585,9 +600,9 @@ int causal_tc_walk(const FlareProblem* p, const void* q, const void* k, const vo
 }  // namespace flare
 
 namespace flare {
-int causal_tc_record(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, float2* rml,
+int causal_tc_record(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, __nv_bfloat16* rlo, float2* rml,
                      int chunks, cudaStream_t st) {
-  return p->D == 32 ? launch_record_tc<32>(p, q, k, v, racc, rml, chunks, st)
-                    : launch_record_tc<64>(p, q, k, v, racc, rml, chunks, st);
+  return p->D == 32 ? launch_record_tc<32>(p, q, k, v, racc, rlo, rml, chunks, st)
+                    : launch_record_tc<64>(p, q, k, v, racc, rlo, rml, chunks, st);
 }
 }  // namespace flare

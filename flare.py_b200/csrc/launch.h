@@ -75,30 +75,31 @@ int tc_set_dyn_smem(const void* kernel, int bytes);
 bool causal_tc_walk_supported(const FlareProblem* p, const void* q, const void* k, const void* v, const void* y);
 // pass 1 for the same shapes: the record of every 128-token chunk on its own, racc [chunks][B][H][M][D] in 16 bits and
 // rml [chunks][B][H][M] = (m, l); the scan turns them into the prefixes in place
-int causal_tc_record(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, float2* rml,
+int causal_tc_record(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* racc, __nv_bfloat16* rlo, float2* rml,
                      int chunks, cudaStream_t st);
 // redo: int [chunks][B*H], written by every CTA: 1 where the chunk must be redone by the fp32 walk.
 // pacc [chunks][B][H][M][D] bf16 and pml [chunks][B][H][M] (m, l): the prefix of every chunk as the scan wrote it.
 int causal_tc_walk(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, const __nv_bfloat16* pacc,
                    const float2* pml, int* redo, int chunks, cudaStream_t st);
 
-// Causal backward on the tensor cores (flare_causal_bwd_tc.cu), same shapes; pacc, pml: the prefixes the forward's scan
-// wrote.  dq32: [B][H][M][D], or [H][M][D] summed over the batch.
+// Causal backward on the tensor cores (flare_causal_bwd_tc.cu), same shapes; pacc + plo, pml: the prefixes the forward's
+// scan wrote.  dq32: [B][H][M][D], or [H][M][D] summed over the batch.
 bool causal_bwd_tc_supported(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
                              const void* dk, const void* dv);
 size_t causal_bwd_tc_workspace(const FlareProblem* p);
 int causal_bwd_tc(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy, const __nv_bfloat16* pacc,
-                  const float2* pml, float* dq32, bool sum_batch, void* dk, void* dv, void* workspace, cudaStream_t st);
+                  const __nv_bfloat16* plo, const float2* pml, float* dq32, bool sum_batch, void* dk, void* dv, void* workspace, cudaStream_t st);
 // the fp32 backward of the (b, h) whose redo flag is set; their dq goes to partial 0 of dq_part, zeros to the others
 int causal_bwd_redo(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
-                    const __nv_bfloat16* pacc, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
+                    const __nv_bfloat16* pacc, const __nv_bfloat16* plo, const float2* pml, const int* redo, float* dq_part, int units, void* dk,
                     void* dv, float* sub, cudaStream_t st);
 // the whole prefill of the tensor-core shapes (flare_causal.cu); redo: int [chunks][B*H]
 int causal_tc_prefill(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, __nv_bfloat16* pacc,
-                      float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st);
-// record and scan passes of the prefill (flare_causal.cu): the prefix of every chunk into pacc, pml
-int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc, float2* pml,
-                     const float* state_in, float* state_out, int chunks, cudaStream_t st);
+                      __nv_bfloat16* plo, float2* pml, int* redo, const float* state_in, float* state_out, cudaStream_t st);
+// record and scan passes of the prefill (flare_causal.cu): the prefix of every chunk into pacc, pml and, unless it is
+// null, the remainders of pacc into plo
+int causal_tc_prefix(const FlareProblem* p, const void* q, const void* k, const void* v, __nv_bfloat16* pacc,
+                     __nv_bfloat16* plo, float2* pml, const float* state_in, float* state_out, int chunks, cudaStream_t st);
 
 // Causal linear attention on the tensor cores (flare_causal_linear_tc.cu): 16-bit inputs, Dk = 128, Dv in {32, 64}.
 bool causal_linear_tc_supported(int B, int H, int N, int Dk, int Dv, int dtype, const void* q, const int64_t* qs,
