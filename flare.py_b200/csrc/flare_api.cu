@@ -491,8 +491,9 @@ int flare_mixer_bwd(const FlareProblem* p, const void* q, const void* k, const v
   float* part = reinterpret_cast<float*>(w);      w += up256(S * rows * p->D * sizeof(float));
   float* dz32 = reinterpret_cast<float*>(w);      w += up256(rows * p->D * sizeof(float));
   float* delta = reinterpret_cast<float*>(w);
-  TRY(flare_bwd_dz_partial(&pp, q, k, dy, key_mask, lse_n, part, stream));
-  TRY(flare_reduce_sum(part, pp.n_splits, (int64_t)rows, p->D, dz32, stream));
+  // one range: its sums are dZ (the launch that would copy them took 12 us of an LRA layer's step)
+  TRY(flare_bwd_dz_partial(&pp, q, k, dy, key_mask, lse_n, S > 1 ? part : dz32, stream));
+  if (S > 1) TRY(flare_reduce_sum(part, pp.n_splits, (int64_t)rows, p->D, dz32, stream));
   TRY(flare_bwd_main(&pp, FLARE_TERM_BOTH, q, k, v, dy, y, key_mask, z32, dz32, lse_m, lse_n, dk, dv, delta, part, stream));
   if (p->q_stride[0] == 0) {
     TRY(flare_reduce_sum(part, pp.n_splits * p->B, (int64_t)p->H * p->M, p->D, dq32, stream));

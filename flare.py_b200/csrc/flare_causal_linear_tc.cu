@@ -122,12 +122,25 @@ k_cl_tc_prefix(const float* __restrict__ sums, T* __restrict__ prefix, int chunk
   const float* s = sums + bh * chunks * per_chunk + e;
   T* p = prefix + bh * chunks * per_chunk + e;
   float r0 = 0.f, r1 = 0.f;
-  float2 nx = *reinterpret_cast<const float2*>(s);
-  for (int c = 0; c < chunks; ++c) {
-    const float2 cur = nx;
-    if (c + 1 < chunks) nx = *reinterpret_cast<const float2*>(s + (long long)(c + 1) * per_chunk);
-    *reinterpret_cast<uint32_t*>(p + (long long)c * per_chunk) = Op16<T>::pack(r0 * inv_n, r1 * inv_n);
-    r0 += cur.x; r1 += cur.y;
+  // the time is the latency of the loads: eight chunks in flight, and the next eight before these are used
+  constexpr int kAhead = 8;
+  float2 nx[kAhead];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      nx[u] = c0 + u < chunks ? *reinterpret_cast<const float2*>(s + (long long)(c0 + u) * per_chunk) : make_float2(0.f, 0.f);
+  };
+  fetch(0);
+  for (int c0 = 0; c0 < chunks; c0 += kAhead) {
+    float2 cur[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) cur[u] = nx[u];
+    if (c0 + kAhead < chunks) fetch(c0 + kAhead);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (c0 + u < chunks) *reinterpret_cast<uint32_t*>(p + (long long)(c0 + u) * per_chunk) = Op16<T>::pack(r0 * inv_n, r1 * inv_n);
+      r0 += cur[u].x; r1 += cur[u].y;
+    }
   }
 }
 

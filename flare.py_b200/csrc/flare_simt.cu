@@ -1146,7 +1146,7 @@ int simt_dq_partial(const Ctx& c, int dtype, const void* q, const void* k, const
 int simt_scatter(const Ctx& c, int dtype, const void* q, const void* k, const float* z32,
                  const uint8_t* mask, void* y, float* lse_n, cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    constexpr int RM = max_rows<kD, 2>();
+    constexpr int RM = kD == 16 ? 2 : max_rows<kD, 2>();             // four rows of 16: 19 us against 16 at two (fp32, N = 4096, 16 heads)
     FLARE_ROWS(RM, c.N, (long long)c.B * c.H, k_scatter_rows<T, kD, kR><<<dim3((c.N + 32 * kR - 1) / (32 * kR), c.H, c.B), kThreads, 0, st>>>(
                             c, (const T*)q, (const T*)k, z32, mask, (T*)y, lse_n))
     else k_scatter<T, kD><<<tok_grid(c), kThreads, 0, st>>>(c, (const T*)q, (const T*)k, z32, mask, (T*)y, lse_n)));

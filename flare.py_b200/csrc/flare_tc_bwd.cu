@@ -394,8 +394,7 @@ k_tc_bwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtens
       tmem_wait_st();
       fence_proxy_async();
       tc_fence_before();
-      __syncthreads();
-      aborted = *reinterpret_cast<volatile int*>(abort_flag) != 0;
+      aborted = __syncthreads_or(*reinterpret_cast<volatile int*>(abort_flag)) != 0;
       if (aborted) break;
 
       if (warp == 0) {
