@@ -183,7 +183,8 @@ int flare_gather_partial(const FlareProblem* p, const void* q, const void* k, co
     const int rc = tc_lat2_supported(c, p->dtype) ? tc_gather_partial2(c, p->dtype, q, k, v, key_mask, rec, (cudaStream_t)stream)
                                                   : tc_gather_partial(c, q, k, v, rec, (cudaStream_t)stream);
     if (rc == FLARE_OK) { ++g_tc_passes; return after_launch("gather_partial (tcgen05)"); }
-    if (rc != FLARE_EUNSUPPORTED) return fail(rc, "gather_partial (tcgen05): launch setup failed");
+    // the fp32 kernels know no dropout
+    if (rc != FLARE_EUNSUPPORTED || p->dropout_p > 0.f) return fail(rc, "gather_partial (tcgen05): launch setup failed");
   }
   ++g_simt_passes;
   TRY(simt_gather_partial(c, p->dtype, q, k, v, key_mask, rec, (cudaStream_t)stream));
@@ -231,7 +232,8 @@ int flare_scatter(const FlareProblem* p, const void* q, const void* k, const flo
     const int rc = tc_scatter2_supported(c, p->dtype) ? tc_scatter2(c, p->dtype, q, k, z32, key_mask, y, lse_n, (cudaStream_t)stream)
                                                       : tc_scatter(c, q, k, z32, key_mask, y, lse_n, (cudaStream_t)stream);
     if (rc == FLARE_OK) { ++g_tc_passes; return after_launch("scatter (tcgen05)"); }
-    if (rc != FLARE_EUNSUPPORTED) return fail(rc, "scatter (tcgen05): launch setup failed");
+    // the fp32 kernels know no dropout
+    if (rc != FLARE_EUNSUPPORTED || p->dropout_p > 0.f) return fail(rc, "scatter (tcgen05): launch setup failed");
   }
   ++g_simt_passes;
   TRY(simt_scatter(c, p->dtype, q, k, z32, key_mask, y, lse_n, (cudaStream_t)stream));
@@ -255,7 +257,8 @@ int flare_bwd_dz_partial(const FlareProblem* p, const void* q, const void* k, co
                        ? tc_dz_partial2(c, p->dtype, q, k, dy, key_mask, lse_n, dz_part, (cudaStream_t)stream)
                        : tc_dz_partial(c, q, k, dy, lse_n, dz_part, (cudaStream_t)stream);
     if (rc == FLARE_OK) { ++g_tc_passes; return after_launch("bwd_dz_partial (tcgen05)"); }
-    if (rc != FLARE_EUNSUPPORTED) return fail(rc, "bwd_dz_partial (tcgen05): launch setup failed");
+    // the fp32 kernels know no dropout
+    if (rc != FLARE_EUNSUPPORTED || p->dropout_p > 0.f) return fail(rc, "bwd_dz_partial (tcgen05): launch setup failed");
   }
   ++g_simt_passes;
   TRY(simt_dz_partial(c, p->dtype, q, k, dy, key_mask, lse_n, dz_part, (cudaStream_t)stream));

@@ -24,6 +24,24 @@ inline EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
+// cuTensorMapEncodeTiled wants a current context, which a thread that has made no runtime call yet (autograd's, in its
+// first backward) does not have: cudaSetDevice makes the device's own context current, also while a stream captures.
+inline CUresult encode_tiled(EncodeTiledFn enc, CUtensorMap* map, int dtype16, const void* base, const cuuint64_t* dims,
+                             const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle sw) {
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  auto call = [&] {
+    return enc(map, dtype16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims,
+               strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = call();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = call();
+  }
+  return r;
+}
+
 // Map of a 16-bit [d3][d2][rows][D] tensor (unit stride on D, byte strides for the others) with a
 // box of {D, box_rows, 1, 1} and the swizzle that matches a row of 2*D bytes.
 // dtype16: 0 = fp16, 1 = bf16.  Returns false when the driver rejects the description.
@@ -35,14 +53,10 @@ inline bool make_tile_map(CUtensorMap* map, const void* base, int dtype16, int D
   cuuint64_t dims[4] = {(cuuint64_t)D, rows, d2, d3};
   cuuint64_t strides[3] = {stride_row_b, stride_d2_b, stride_d3_b};
   cuuint32_t box[4] = {(cuuint32_t)D, box_rows, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
   const int rowb = 2 * D;
   CUtensorMapSwizzle sw = rowb == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
                           : rowb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-  CUresult r = enc(map, dtype16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return encode_tiled(enc, map, dtype16, base, dims, strides, box, sw) == CUDA_SUCCESS;
 }
 
 // Same tensor, but a box of `box_cols` of its D columns (a multiple of 8; 2 * box_cols bytes per tile row, which picks the
@@ -55,15 +69,11 @@ inline bool make_tile_map_cols(CUtensorMap* map, const void* base, int dtype16, 
   cuuint64_t dims[4] = {(cuuint64_t)D, rows, d2, d3};
   cuuint64_t strides[3] = {stride_row_b, stride_d2_b, stride_d3_b};
   cuuint32_t box[4] = {(cuuint32_t)box_cols, box_rows, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
   const int rowb = 2 * box_cols;
   if (rowb != 32 && rowb != 64 && rowb != 128) return false;
   CUtensorMapSwizzle sw = rowb == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
                           : rowb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-  CUresult r = enc(map, dtype16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return encode_tiled(enc, map, dtype16, base, dims, strides, box, sw) == CUDA_SUCCESS;
 }
 
 }  // namespace flare

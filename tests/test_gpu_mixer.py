@@ -445,3 +445,25 @@ def test_general_backward_in_64_latent_steps(fb, cuda_dev, dtype, N, M):
     y.backward(dy.float())
     # two correct 16-bit evaluations differ by a few roundings of the operands (bf16: 2^-9 each)
     assert_close(got, [y.detach(), qf.grad, kf.grad, vf.grad], 1e-2 if dtype == torch.bfloat16 else 2e-3)
+
+
+def test_a_fresh_thread_runs_the_tensor_core_kernels(fb, cuda_dev):
+    """A thread whose first CUDA work is ours (autograd's, in the first backward) has no current context yet: the tensor
+    maps must be made all the same, not the fp32 kernels be taken."""
+    import threading
+    q, k, v, _ = (t.to(cuda_dev) for t in O.make_inputs(1, 2, 700, 64, 16, dtype=torch.bfloat16, seed=5))
+    want = fb.flare_multihead_mixer(q, k, v, 1.0)
+    torch.cuda.synchronize()
+    got = []
+
+    def work():
+        with torch.no_grad():
+            got.append(fb.flare_multihead_mixer(q, k, v, 1.0))
+
+    tc0, simt0 = fb.pass_counts()
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    tc1, simt1 = fb.pass_counts()
+    assert (tc1 - tc0, simt1 - simt0) == (2, 0)
+    assert torch.equal(got[0], want)
