@@ -707,6 +707,7 @@ k_dq_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* __re
     __syncthreads();
     int lo, hi;
     quarter<1>(cnt, warp, lo, hi);
+#pragma unroll 2
     for (int j = lo; j < hi; ++j) {
       const float c2 = sC2[j];
       if (c2 == -INFINITY) continue;               // the same for the whole warp
@@ -903,6 +904,7 @@ k_bwd_tokens_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const
     __syncthreads();
     int lo, hi;
     quarter<1>(cnt, warp, lo, hi);
+#pragma unroll 2
     for (int j = lo; j < hi; ++j) {
       float2 qr[D / 2], x[D / 2];
       float s[R], dS[R];
@@ -1158,7 +1160,7 @@ int simt_bwd_tokens(const Ctx& c, int dtype, const void* q, const void* k, const
                     const float* lse_m, const float* lse_n, void* dk, void* dv, float* delta_n,
                     cudaStream_t st) {
   FLARE_DISPATCH_T(dtype, FLARE_DISPATCH_D(c.D,
-    constexpr int RM = max_rows<kD, 5>();
+    constexpr int RM = kD == 8 ? 2 : max_rows<kD, 5>();
     FLARE_ROWS(RM, c.N, (long long)c.B * c.H, k_bwd_tokens_rows<T, kD, kR><<<dim3((c.N + 32 * kR - 1) / (32 * kR), c.H, c.B), kThreads, 0, st>>>(
                             c, (const T*)q, (const T*)k, (const T*)v, (const T*)dy, (const T*)y, mask, z32, dz32, lse_m, lse_n,
                             (T*)dk, (T*)dv, delta_n))
