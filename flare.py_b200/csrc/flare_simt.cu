@@ -1100,7 +1100,7 @@ static inline dim3 tok_grid(const Ctx& c) {
 // Rows per lane of the register-blocked kernels (0: one row per thread is the better form -- wide rows, whose
 // operands leave no registers for a second one).  kArrays: D-wide register arrays per row.
 template <int D, int kArrays> constexpr int max_rows() {
-  return 4 * D * kArrays <= 160 ? 4 : 2 * D * kArrays <= 160 ? 2 : 0;
+  return 4 * D * kArrays <= 160 ? 4 : 2 * D * kArrays <= 160 ? 2 : D <= 32 && D * kArrays <= 128 ? 1 : 0;
 }
 // Launch with R rows per lane, R <= RM: no more than the rows fill (a block takes 32 R of them), and no more than
 // leaves one and a half blocks per SM (`others_` blocks run per block of rows).
@@ -1108,7 +1108,7 @@ template <int D, int kArrays> constexpr int max_rows() {
   if constexpr (RM_ > 0) {                                                       \
     const long long r32 = ((rows_) + 31) / 32, least = 3LL * num_sms() / 2;          \
     if (RM_ >= 4 && r32 > 2 && (r32 + 3) / 4 * (others_) >= least) { constexpr int kR = RM_ >= 4 ? 4 : 1; __VA_ARGS__; } \
-    else if (r32 > 1 && (r32 + 1) / 2 * (others_) >= least) { constexpr int kR = 2; __VA_ARGS__; } \
+    else if (RM_ >= 2 && r32 > 1 && (r32 + 1) / 2 * (others_) >= least) { constexpr int kR = RM_ >= 2 ? 2 : 1; __VA_ARGS__; } \
     else                          { constexpr int kR = 1; __VA_ARGS__; }         \
     return FLARE_OK;                                                             \
   }
