@@ -57,7 +57,7 @@ double split_cost(const FlareProblem* p, bool tc, long long tiles, long long S) 
   const long long bh = (long long)p->B * p->H, nb = (p->M + 127) / 128, per = (tiles + S - 1) / S;
   const double parts = (double)S * bh * p->M * (p->D + 2) * 4 * 3 / 2.5e6;          // partial records written and read again
   if (!tc) {                                                                        // fp32 kernels: about two blocks per SM
-    const long long lpb = p->D == 8 ? 128 : p->D == 16 ? 64 : 32;       // latents per block of the widest pass
+    const long long lpb = p->D == 8 ? 128 : 64;       // latents per block of most passes
     const long long grid = bh * ((p->M + lpb - 1) / lpb) * S;
     return (double)((grid + 295) / 296) * (per + 0.3) * 4 + parts;
   }
