@@ -514,6 +514,18 @@ Tensor triple_contract(const Tensor& t, int x, int y, int z, const Tensor& a, co
   return out;
 }
 
+// The kernels take every size from one operand and index the others and the rank-3 tensor by it: q1 and q2 must agree in
+// heads and tokens, so must k1, k2 and v, and q1, q2, k1, k2 in features.
+void check_triple(const Tensor& q1, const Tensor& q2, const Tensor& k1, const Tensor& k2, const Tensor& v) {
+  for (const Tensor* t : {&q1, &q2, &k1, &k2, &v})
+    if (t->dim() != 4) raise_py(PyExc_ValueError, "q1, q2, k1, k2, v must be [B,H,N,D]");
+  auto rows = [](const Tensor& a, const Tensor& b) { return a.size(0) * a.size(1) == b.size(0) * b.size(1) && a.size(2) == b.size(2); };
+  if (!rows(q1, q2) || !rows(k1, k2) || !rows(k1, v) || q1.size(0) * q1.size(1) != k1.size(0) * k1.size(1))
+    raise_py(PyExc_ValueError, "q1, q2 (and k1, k2, v) must agree in batch, heads and tokens");
+  for (const Tensor* t : {&q2, &k1, &k2})
+    if (t->size(3) != q1.size(3)) raise_py(PyExc_ValueError, "q1, q2, k1, k2 must share a feature dimension");
+}
+
 class TripleFn : public torch::autograd::Function<TripleFn> {
  public:
   static variable_list forward(AutogradContext* ctx, const Tensor& q1, const Tensor& q2, const Tensor& k1, const Tensor& k2,
@@ -521,6 +533,7 @@ class TripleFn : public torch::autograd::Function<TripleFn> {
     at::AutoDispatchBelowADInplaceOrView below;
     for (const Tensor* t : {&q1, &q2, &k1, &k2, &v}) need_cuda(*t);
     same_dtype("q1, q2, k1, k2, v must share a dtype", {&q1, &q2, &k1, &k2, &v});
+    check_triple(q1, q2, k1, k2, v);
     c10::cuda::CUDAGuard guard(v.device());
     const int64_t B = q1.size(0), H = q1.size(1), N = q1.size(2), Dq = q1.size(3), Dv = v.size(3);
     const Tensor fq1 = flat(q1), fq2 = flat(q2), fk1 = flat(k1), fk2 = flat(k2), fv = flat(v);

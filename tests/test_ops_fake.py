@@ -67,3 +67,23 @@ def test_autocast_casts_the_latents_like_sdpa(monkeypatch):
             fb.flare_multihead_mixer(q, k.float(), v.float(), dropout_p=0.1)      # fp32 has no dropout kernels
         with pytest.raises(ValueError):
             fb.flare_multihead_mixer(q.half(), k, v, dropout_p=1.0)
+
+
+@pytest.mark.parametrize("which,shape", [
+    (1, (1, 2, 64, 32)),     # q2 wider than k2: the contraction would read past STATE
+    (1, (1, 2, 64, 8)),      # q2 narrower
+    (3, (1, 2, 64, 32)),     # k2 wider than q2
+    (0, (1, 2, 64, 32)),     # q1 wider than k1
+    (2, (1, 2, 64, 32)),     # k1 wider than q1
+    (1, (1, 2, 48, 16)),     # fewer tokens than q1
+    (4, (1, 2, 48, 16)),     # fewer tokens than k1
+    (4, (1, 1, 64, 16)),     # fewer heads
+    (3, (2, 64, 16)),        # three dimensions
+])
+def test_triple_attention_refuses_mismatched_sizes_before_any_launch(which, shape):
+    """The refusal comes from the host's size check: nothing is allocated or launched before it."""
+    shapes = [(1, 2, 64, 16)] * 5
+    shapes[which] = shape
+    with FakeTensorMode():
+        with pytest.raises(ValueError):
+            fb.triple_attention(*(torch.empty(s, dtype=torch.float16, device="cuda") for s in shapes))
