@@ -373,7 +373,7 @@ Four mixer_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, doubl
                         double dropout_p, int64_t dropout_seed) {
   if (!at::GradMode::is_enabled() || !(q.requires_grad() || k.requires_grad() || v.requires_grad())) {
     at::AutoDispatchBelowADInplaceOrView below;
-    return Op_mixer_fwd::get().call(as_dtype(q, k.scalar_type()), k, v, scale, key_mask, dropout_p, dropout_seed);
+    return Op_mixer_fwd::get().call(q, k, v, scale, key_mask, dropout_p, dropout_seed);
   }
   auto r = MixerFn::apply(q, k, v, scale, key_mask, dropout_p, dropout_seed);
   return {r[0], r[1], r[2], r[3]};
@@ -628,7 +628,13 @@ FLARE_PY(mixer, 7, {
   const int64_t seed = int_arg(a[6]);
   need_cuda(q); need_cuda(k); need_cuda(v);
   Tensor y;
-  { pybind11::gil_scoped_release nogil; y = std::get<0>(Op_mixer_fwd::get().call(q, k, v, scale, mask, p, seed)); }
+  {
+    pybind11::gil_scoped_release nogil;
+    // fp32 latents under autocast: MixerFn rounds them where a gradient is wanted.  The other calls round them here, since
+    // the autograd kernel does not run on inference tensors or in inference mode.
+    const bool grad = at::GradMode::is_enabled() && q.requires_grad();
+    y = std::get<0>(Op_mixer_fwd::get().call(grad ? q : as_dtype(q, k.scalar_type()), k, v, scale, mask, p, seed));
+  }
   return THPVariable_Wrap(std::move(y));
 })
 FLARE_PY(causal_prefill, 5, {

@@ -260,3 +260,42 @@ def test_fp16_autocast_with_grad_scaler_takes_a_step(fb, cuda_dev):
     scaler.step(opt)
     scaler.update()
     assert not torch.equal(before, model.blocks[0].att.latent_q.detach())
+
+
+# ---------------------------------------------------------------------------------------------------------
+# evaluation of a trained model: fp32 parameters, autocast, inference mode
+# ---------------------------------------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("which", ["FLARE", "FLAREBlock", "FLAREModel", "LraFLARE", "LraFLAREBlock"])
+def test_modules_under_inference_mode_and_autocast(fb, cuda_dev, which, dtype):
+    """The same kernels on the same operands as under no_grad: equal bits."""
+    torch.manual_seed(3)
+    own = {"LraFLARE": dict(kv_proj_hidden_dim=64), "LraFLAREBlock": dict(kv_proj_hidden_dim=64, ffn_hidden_dim=64)}.get(which, {})
+    if which == "FLAREModel":
+        m, x = fb.FLAREModel(3, 2, channel_dim=64, num_blocks=2, num_heads=4, num_latents=32), torch.randn(2, 300, 3)
+    else:
+        m, x = getattr(fb.modules, which)(64, num_heads=4, num_latents=32, **own), torch.randn(2, 300, 64)
+    m, x = m.to(cuda_dev).eval(), x.to(cuda_dev)
+    with torch.autocast("cuda", dtype=dtype):
+        with torch.no_grad():
+            want = m(x)
+        with torch.inference_mode():
+            got = m(x)
+    first = lambda o: o[0] if isinstance(o, tuple) else o
+    assert torch.equal(first(got), first(want))
+
+
+@pytest.mark.gpu
+def test_mixer_on_inference_tensors_under_autocast(fb, cuda_dev):
+    g = torch.Generator().manual_seed(5)
+    q, k, v = (torch.randn(*s, generator=g).to(cuda_dev) for s in ((2, 32, 16), (1, 2, 200, 16), (1, 2, 200, 16)))
+    k, v = k.bfloat16(), v.bfloat16()
+    with torch.inference_mode():
+        made = [t.clone() for t in (q, k, v)]
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = fb.flare_multihead_mixer(q, k, v)
+        got = fb.flare_multihead_mixer(*made)                 # inference tensors outside inference mode
+        kept = fb.flare_multihead_mixer(q.requires_grad_(True), k, v).detach()
+    assert got.dtype == torch.bfloat16
+    assert torch.equal(got, want) and torch.equal(kept, want)

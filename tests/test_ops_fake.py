@@ -4,6 +4,7 @@ are called directly here; differentiation end to end is covered by the GPU tests
 import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 import flare_b200 as fb
 
@@ -67,6 +68,30 @@ def test_autocast_casts_the_latents_like_sdpa(monkeypatch):
             fb.flare_multihead_mixer(q, k.float(), v.float(), dropout_p=0.1)      # fp32 has no dropout kernels
         with pytest.raises(ValueError):
             fb.flare_multihead_mixer(q.half(), k, v, dropout_p=1.0)
+
+
+@pytest.mark.parametrize("inference,requires_grad", [(True, True), (True, False), (False, False)])
+def test_latents_meet_the_operator_in_the_autocast_dtype(monkeypatch, inference, requires_grad):
+    """No gradient wanted: the operator's backend kernel gets q rounded, also in inference mode and for inference tensors,
+    where the operator's autograd kernel does not run."""
+    monkeypatch.setattr(torch, "is_autocast_enabled", lambda *a: True)
+    monkeypatch.setattr(torch, "get_autocast_dtype", lambda *a: torch.bfloat16)
+    seen = []
+
+    class Record(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func is torch.ops.flare_b200.mixer_fwd.default:
+                seen.append(tuple(a.dtype for a in args[:3]))
+            return func(*args, **(kwargs or {}))
+
+    with FakeTensorMode():
+        with torch.inference_mode():
+            q, k = (torch.empty(s, device="cuda", dtype=dt) for s, dt in (((2, 8, 16), torch.float32), ((1, 2, 64, 16), torch.bfloat16)))
+        if requires_grad:
+            q = torch.empty(2, 8, 16, device="cuda", requires_grad=True)
+        with torch.inference_mode(inference), Record():
+            y = fb.flare_multihead_mixer(q, k, k)
+    assert y.dtype == torch.bfloat16 and seen == [(torch.bfloat16,) * 3]
 
 
 @pytest.mark.parametrize("which,shape", [
