@@ -453,7 +453,8 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
     const auto s = ctx->get_saved_variables();
     const Tensor &q_ = s[0], &saved = s[3];
     c10::cuda::CUDAGuard guard(s[1].device());
-    const Tensor q = latents(q_), k = tok(s[1]), v = tok(s[2]), dy = tok(g[0]);
+    // a batch made by expand() is a batch here: its entries have gradients of their own, which autograd folds back itself
+    const Tensor q = tok(q_), k = tok(s[1]), v = tok(s[2]), dy = tok(g[0]);
     FlareProblem p = problem(q, k, ctx->saved_data["scale"].toDouble());
     Tensor dk = at::detail::empty_cuda(k.sizes(), k.options()), dv = at::detail::empty_cuda(v.sizes(), v.options());
     set_stride(p.v_stride, v);
@@ -461,27 +462,19 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
     set_stride(p.dk_stride, dk);
     set_stride(p.dv_stride, dv);
     const flare_stream_t st = stream_of(k);
-    const bool shared = q_.dim() == 3;
     Tensor dq;
     if (saved.defined()) {
       dq = f32(q.sizes(), k);
       const Tensor ws = scratch(flare_causal_train_bwd_workspace_bytes(&p), k);
       check_rc(flare_causal_train_bwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), dy.data_ptr(), saved.data_ptr(), fp(dq),
                                       dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), st), "flare_causal_train_bwd");
-      // a batch made by expand(): autograd sums over it, so the whole gradient goes to its first entry's share
-      if (!shared && q.dim() == 3) {
-        Tensor full = at::zeros(q_.sizes(), dq.options());
-        full.select(0, 0).copy_(dq);
-        dq = full;
-      }
     } else {
       dq = f32({p.B, p.H, p.M, p.D}, k);
       const Tensor ws = scratch(flare_causal_bwd_workspace_bytes(&p), k);
       check_rc(flare_causal_bwd(&p, q.data_ptr(), k.data_ptr(), v.data_ptr(), dy.data_ptr(), fp(dq), dk.data_ptr(),
                                 dv.data_ptr(), fp(ws), st), "flare_causal_bwd");
-      // one latent gradient per (b, h): shared latents sum over the batch; a batch made by expand() gets the
-      // per-batch gradients, which autograd folds back itself
-      if (shared) {
+      // one latent gradient per (b, h): shared latents sum over the batch
+      if (q.dim() == 3) {
         Tensor sum = f32({p.H, p.M, p.D}, k);
         check_rc(flare_reduce_sum(fp(dq), p.B, (int64_t)p.H * p.M, p.D, fp(sum), st), "flare_reduce_sum");
         dq = sum;

@@ -363,6 +363,27 @@ def test_training_step_with_shared_latents(cuda_dev):
     assert O.rel_l2(vd.grad.double().cpu(), vr.grad) <= 1e-4
 
 
+@pytest.mark.parametrize("dtype,M,tol", [(torch.bfloat16, 32, 5e-3), (torch.bfloat16, 160, 3e-2), (torch.float32, 32, 1e-4)])
+def test_gradient_of_batch_expanded_latents(cuda_dev, dtype, M, tol):
+    """One latent set expand()-ed over the batch and differentiated itself: every batch entry has its own gradient (on
+    the tensor-core shapes and on the others), and the set below it gets their sum."""
+    import flare_b200 as fb
+    B, H, N, D = 3, 2, 300, 32
+    q, k, v, dy = O.make_inputs(B, H, N, M, D, dtype=dtype, seed=33)
+    q1 = q.to(cuda_dev).requires_grad_(True)
+    qe = q1.unsqueeze(0).expand(B, -1, -1, -1)
+    kd, vd = k.to(cuda_dev).requires_grad_(True), v.to(cuda_dev).requires_grad_(True)
+    y = fb.flare_causal_mixer(qe, kd, vd, 1.0)
+    got = torch.autograd.grad(y, (qe, q1, kd, vd), dy.to(cuda_dev))
+    qf = q.double().unsqueeze(0).repeat(B, 1, 1, 1)
+    dq, dk, dv = O.causal_bwd_chunked(qf, *(t.double() for t in (k, v, dy)), 1.0, chunk=64)
+    assert got[0].shape == dq.shape
+    for b in range(B):
+        assert O.rel_l2(got[0][b].double().cpu(), dq[b]) <= tol
+    for g, r in zip(got[1:], (dq.sum(0), dk, dv)):
+        assert O.rel_l2(g.double().cpu(), r) <= tol
+
+
 def test_decode_step_replays_from_a_cuda_graph(cuda_dev):
     """The serving loop: one decode step recorded in a CUDA graph over static k_t, v_t, y_t buffers and the
     state record, replayed once per token (the state lives in one fp32 tensor updated in place, so the
