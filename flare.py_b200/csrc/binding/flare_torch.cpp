@@ -16,6 +16,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 #include <torch/library.h>
@@ -378,6 +380,45 @@ Four mixer_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, doubl
   auto r = MixerFn::apply(q, k, v, scale, key_mask, dropout_p, dropout_seed);
   return {r[0], r[1], r[2], r[3]};
 }
+// The backward operators have no derivative of their own: where a graph of them is recorded (create_graph), differentiating
+// their results raises instead of leaving their share out.
+template <typename... In>
+Three no_second_derivative(const char* name, Three r, const In&... in) {
+  if (torch::autograd::compute_requires_grad(in...)) {
+    const std::shared_ptr<torch::autograd::Node> node(
+        new torch::autograd::NotImplemented(name, torch::autograd::collect_next_edges(in...)), torch::autograd::deleteNode);
+    for (const Tensor& t : {std::get<0>(r), std::get<1>(r), std::get<2>(r)}) torch::autograd::set_history(t, node);
+  }
+  return r;
+}
+Three mixer_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& dy, const Tensor& y,
+                         const Tensor& z32, const Tensor& lse_m, const Tensor& lse_n, double scale,
+                         const optional<Tensor>& key_mask, double dropout_p, int64_t dropout_seed) {
+  Three r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = Op_mixer_bwd::get().call(q, k, v, dy, y, z32, lse_m, lse_n, scale, key_mask, dropout_p, dropout_seed);
+  }
+  return no_second_derivative("flare_b200::mixer_bwd", std::move(r), q, k, v, dy, y, z32, lse_m, lse_n);
+}
+Three gather_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& dz, const Tensor& z32,
+                          const Tensor& lse_m, double scale, const optional<Tensor>& key_mask) {
+  Three r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = Op_gather_bwd::get().call(q, k, v, dz, z32, lse_m, scale, key_mask);
+  }
+  return no_second_derivative("flare_b200::gather_bwd", std::move(r), q, k, v, dz, z32, lse_m);
+}
+Three scatter_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& z, const Tensor& dy, const Tensor& y,
+                           const Tensor& lse_n, double scale, const optional<Tensor>& key_mask) {
+  Three r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = Op_scatter_bwd::get().call(q, k, z, dy, y, lse_n, scale, key_mask);
+  }
+  return no_second_derivative("flare_b200::scatter_bwd", std::move(r), q, k, z, dy, y, lse_n);
+}
 Three gather_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const optional<Tensor>& key_mask) {
   auto r = GatherFn::apply(q, k, v, scale, key_mask);
   return {r[0], r[1], r[2]};
@@ -697,6 +738,9 @@ TORCH_LIBRARY_IMPL(flare_b200, CUDA, m) {
   m.impl("scatter_bwd", &scatter_bwd);
 }
 TORCH_LIBRARY_IMPL(flare_b200, Autograd, m) {
+  m.impl("scatter_bwd", &scatter_bwd_autograd);
+  m.impl("gather_bwd", &gather_bwd_autograd);
+  m.impl("mixer_bwd", &mixer_bwd_autograd);
   m.impl("mixer_fwd", &mixer_fwd_autograd);
   m.impl("gather_fwd", &gather_fwd_autograd);
   m.impl("scatter_fwd", &scatter_fwd_autograd);

@@ -467,3 +467,22 @@ def test_a_fresh_thread_runs_the_tensor_core_kernels(fb, cuda_dev):
     tc1, simt1 = fb.pass_counts()
     assert (tc1 - tc0, simt1 - simt0) == (2, 0)
     assert torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("which", ["mixer", "gather", "scatter"])
+def test_second_derivatives_raise(cuda_dev, which):
+    """create_graph records the backward operators; using their results is fine, differentiating them is refused (they
+    have no derivative) and never leaves their share of a second-order gradient out in silence."""
+    import flare_b200 as fb
+    B, H, N, M, D = 1, 2, 130, 16, 16
+    g = torch.Generator().manual_seed(3)
+    x = [torch.randn(*s, generator=g).to(cuda_dev).requires_grad_(True)
+         for s in ((H, M, D), (B, H, N, D), (B, H, M, D) if which == "scatter" else (B, H, N, D))]
+    y = {"mixer": fb.flare_multihead_mixer, "gather": lambda *t: fb.flare_gather(*t)[0], "scatter": fb.flare_scatter}[which](*x)
+    plain = torch.autograd.grad(y.square().sum(), x, retain_graph=True)
+    first = torch.autograd.grad(y.square().sum(), x, create_graph=True)
+    for a, b in zip(first, plain):
+        assert a.requires_grad and torch.equal(a.detach(), b)
+    for a in first:
+        with pytest.raises(RuntimeError, match="not implemented"):
+            torch.autograd.grad(a.square().sum(), x, retain_graph=True, allow_unused=True)
