@@ -528,7 +528,12 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
 // ------------------------------------------------------------------------------------------------
 // triple attention and causal linear attention
 // ------------------------------------------------------------------------------------------------
-Tensor flat(const Tensor& t) { return t.reshape({t.size(0) * t.size(1), t.size(2), t.size(3)}).contiguous(); }
+Tensor flat(const Tensor& t) {
+  return t.dim() == 3 ? t : t.reshape({t.size(0) * t.size(1), t.size(2), t.size(3)}).contiguous();
+}
+// What the backward keeps of an input: the input itself where flat() is a view of it (made here, that view would not
+// share its version counter, and a change in place before the backward would go unnoticed), else flat()'s copy.
+Tensor keep(const Tensor& t, const Tensor& flat_t) { return flat_t.is_alias_of(t) ? t : flat_t; }
 
 Tensor triple_outer(const Tensor& a, const Tensor& b, const Tensor& c, double alpha) {
   const int BH = (int)a.size(0), N = (int)a.size(1), Da = (int)a.size(2), Db = (int)b.size(2), Dc = (int)c.size(2);
@@ -573,16 +578,18 @@ class TripleFn : public torch::autograd::Function<TripleFn> {
     const Tensor fq1 = flat(q1), fq2 = flat(q2), fk1 = flat(k1), fk2 = flat(k2), fv = flat(v);
     const Tensor state = triple_outer(fk1, fv, fk2, 1.0 / (double)N);                 // [BH, Dq, Dv, Dq]
     const Tensor o = triple_contract(state, 1, 0, 2, fq1, fq2, 1.0);                  // x = j, y = i, z = k
-    ctx->save_for_backward({fq1, fq2, fk1, fk2, fv, state});
+    const Tensor out = state.view({B, H, Dq, Dv, Dq});       // kept as the output it is: changing it in place is noticed too
+    ctx->save_for_backward({keep(q1, fq1), keep(q2, fq2), keep(k1, fk1), keep(k2, fk2), keep(v, fv), out});
     ctx->saved_data["B"] = B;
     ctx->saved_data["H"] = H;
     ctx->set_materialize_grads(false);             // a loss on O alone adds no zero tensor to dSTATE
-    return {state.view({B, H, Dq, Dv, Dq}), o.view({B, H, N, Dv})};
+    return {out, o.view({B, H, N, Dv})};
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
     if (!g[0].defined() && !g[1].defined()) return variable_list(5);
     const auto s = ctx->get_saved_variables();
-    const Tensor &fq1 = s[0], &fq2 = s[1], &fk1 = s[2], &fk2 = s[3], &fv = s[4], &state = s[5];
+    const Tensor fq1 = flat(s[0]), fq2 = flat(s[1]), fk1 = flat(s[2]), fk2 = flat(s[3]), fv = flat(s[4]);
+    const Tensor state = s[5].flatten(0, 1);
     const int64_t B = ctx->saved_data["B"].toInt(), H = ctx->saved_data["H"].toInt();
     const int64_t N = fq1.size(1), Dq = fq1.size(2), Dv = fv.size(2);
     c10::cuda::CUDAGuard guard(fv.device());

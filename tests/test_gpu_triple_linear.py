@@ -156,3 +156,29 @@ def test_causal_linear_strided_views(cuda_dev):
     y = fb.causal_linear(q, k, v)
     y_ref = O.causal_linear(q.double().cpu(), k.double().cpu(), v.double().cpu())
     assert O.rel_l2(y.double().cpu(), y_ref.double()) <= 1e-5
+
+
+@pytest.mark.parametrize("which", ["state", 0, 1, 2, 3, 4])
+def test_triple_notices_a_change_in_place_before_its_backward(cuda_dev, which):
+    """The backward reads the inputs (contiguous ones without a copy) and STATE: changing one of them in between raises."""
+    import flare_b200 as fb
+    x = [_rand((1, 2, 100, 16), torch.float32, i).to(cuda_dev).requires_grad_(True) for i in range(5)]
+    state, o = fb.triple_attention(*x)
+    with torch.no_grad():
+        (state if which == "state" else x[which]).mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(o.sum(), x)
+
+
+def test_triple_keeps_its_own_copy_of_inputs_it_cannot_view(cuda_dev):
+    """A transposed [B,N,H,D] input is copied in the forward; changing it afterwards does not reach the backward."""
+    import flare_b200 as fb
+    x = [_rand((1, 100, 2, 16), torch.float32, i).to(cuda_dev).transpose(1, 2).requires_grad_(True) for i in range(5)]
+    w = _rand((1, 2, 100, 16), torch.float32, 9).to(cuda_dev)
+    want = torch.autograd.grad((fb.triple_attention(*x)[1] * w).sum(), x)
+    o = fb.triple_attention(*x)[1]
+    with torch.no_grad():
+        for t in x:
+            t.zero_()
+    for a, b in zip(torch.autograd.grad((o * w).sum(), x), want):
+        assert torch.equal(a, b)
