@@ -465,7 +465,9 @@ Tensor causal_decode(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
 
 class CausalFn : public torch::autograd::Function<CausalFn> {
  public:
-  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
+  // train: a gradient is wanted (asked by the caller: nothing requires one in here).  Without, it is the plain prefill: the
+  // training forward takes 294 us where that takes 230 (B = 4, H = 16, N = 8192, M = 128, D = 64).
+  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale, bool train) {
     at::AutoDispatchBelowADInplaceOrView below;
     for (const Tensor* t : {&q_, &k_, &v_}) need_cuda(*t);
     same_dtype("q, k, v must share a dtype", {&q_, &k_, &v_});
@@ -475,7 +477,7 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
     FlareProblem p = problem(q, k, scale);
     // the tensor-core shapes keep the chunk-start states for the backward (M (4 D + 8) bytes per 128 tokens and head);
     // the others rebuild them there
-    const size_t bytes = flare_causal_train_bytes(&p);
+    const size_t bytes = train ? flare_causal_train_bytes(&p) : 0;
     Tensor y, saved;
     if (bytes) {
       y = at::detail::empty_cuda(k.sizes(), k.options());
@@ -521,7 +523,7 @@ class CausalFn : public torch::autograd::Function<CausalFn> {
         dq = sum;
       }
     }
-    return {as_dtype(dq, q_.scalar_type()), dk, dv, Tensor()};
+    return {as_dtype(dq, q_.scalar_type()), dk, dv, Tensor(), Tensor()};
   }
 };
 
@@ -697,7 +699,8 @@ FLARE_PY(causal_mixer, 4, {
   const Tensor &q = tensor_arg(a[0]), &k = tensor_arg(a[1]), &v = tensor_arg(a[2]);
   const double scale = double_arg(a[3]);
   Tensor y;
-  { pybind11::gil_scoped_release nogil; y = CausalFn::apply(q, k, v, scale); }
+  const bool train = torch::autograd::compute_requires_grad(q, k, v);
+  { pybind11::gil_scoped_release nogil; y = CausalFn::apply(q, k, v, scale, train); }
   return THPVariable_Wrap(std::move(y));
 })
 FLARE_PY(triple, 5, {

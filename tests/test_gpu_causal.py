@@ -287,6 +287,23 @@ def test_backward_hands_wide_heads_to_the_fp32_kernel(cuda_dev):
             assert O.rel_l2(g.double().cpu(), r) <= 5e-3, h
 
 
+def test_mixer_without_gradients_is_the_plain_prefill(cuda_dev):
+    """No gradient wanted: the kernels of the prefill, to the bit (the training forward keeps its chunk prefixes in two terms)."""
+    fb = _fb()
+    q, k, v, dy = (t.to(cuda_dev) for t in O.make_inputs(2, 4, 2000, 128, 64, dtype=torch.bfloat16, seed=24))
+    want, _ = fb.flare_causal_prefill(q, k, v, 1.0)
+    assert torch.equal(fb.flare_causal_mixer(q, k, v, 1.0), want)
+    q.requires_grad_(True)
+    with torch.no_grad():
+        assert torch.equal(fb.flare_causal_mixer(q, k, v, 1.0), want)
+    with torch.inference_mode():
+        assert torch.equal(fb.flare_causal_mixer(q, k, v, 1.0), want)
+    y = fb.flare_causal_mixer(q, k, v, 1.0)                  # a gradient for q alone: the training forward
+    dq, = torch.autograd.grad(y, q, dy)
+    ref, _, _ = O.causal_bwd_chunked(*(t.detach().double().cpu() for t in (q, k, v, dy)), 1.0, chunk=128)
+    assert O.rel_l2(dq.double().cpu(), ref) <= 5e-3
+
+
 def test_backward_with_growing_logits(cuda_dev):
     """Keys whose norm grows along the sequence: the running maxima rise by tens of units from chunk to
     chunk, so the carried suffix state is rescaled by tiny factors and early tokens' weights underflow
