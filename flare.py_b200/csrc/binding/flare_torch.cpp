@@ -307,6 +307,7 @@ optional<Tensor> maybe(const Tensor& t) { return t.defined() ? optional<Tensor>(
 
 class MixerFn : public torch::autograd::Function<MixerFn> {
  public:
+  static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
   static variable_list forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k, const Tensor& v, double scale,
                                const optional<Tensor>& key_mask, double dropout_p, int64_t dropout_seed) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -317,8 +318,8 @@ class MixerFn : public torch::autograd::Function<MixerFn> {
     ctx->saved_data["p"] = dropout_p;
     ctx->saved_data["seed"] = dropout_seed;
     ctx->saved_data["qdt"] = (int64_t)q_.scalar_type();
-    // z32, lse_m, lse_n are the backward's operands, not results anyone differentiates: no zero gradients for them
-    ctx->mark_non_differentiable({z32, lse_m, lse_n});
+    // z32, lse_m, lse_n are the backward's operands, not results anyone differentiates: no zero gradients for them (compiled
+    // autograd refuses a function that marks outputs as non-differentiable)
     ctx->set_materialize_grads(false);
     return {y, z32, lse_m, lse_n};
   }
@@ -333,13 +334,13 @@ class MixerFn : public torch::autograd::Function<MixerFn> {
 
 class GatherFn : public torch::autograd::Function<GatherFn> {
  public:
+  static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale,
                                const optional<Tensor>& key_mask) {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [z, z32, lse_m] = Op_gather_fwd::get().call(q, k, v, scale, key_mask);
     ctx->save_for_backward({q, k, v, z32, lse_m, key_mask.value_or(Tensor())});
     ctx->saved_data["scale"] = scale;
-    ctx->mark_non_differentiable({z32, lse_m});
     ctx->set_materialize_grads(false);
     return {z, z32, lse_m};
   }
@@ -353,13 +354,13 @@ class GatherFn : public torch::autograd::Function<GatherFn> {
 
 class ScatterFn : public torch::autograd::Function<ScatterFn> {
  public:
+  static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& z, double scale,
                                const optional<Tensor>& key_mask) {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [y, lse_n] = Op_scatter_fwd::get().call(q, k, z, scale, key_mask);
     ctx->save_for_backward({q, k, z, y, lse_n, key_mask.value_or(Tensor())});
     ctx->saved_data["scale"] = scale;
-    ctx->mark_non_differentiable({lse_n});
     ctx->set_materialize_grads(false);
     return {y, lse_n};
   }

@@ -486,3 +486,30 @@ def test_second_derivatives_raise(cuda_dev, which):
     for a in first:
         with pytest.raises(RuntimeError, match="not implemented"):
             torch.autograd.grad(a.square().sum(), x, retain_graph=True, allow_unused=True)
+
+
+@pytest.mark.parametrize("which", ["mixer", "masked", "autocast", "gather", "scatter"])
+def test_backward_under_compiled_autograd(cuda_dev, which):
+    """torch's compiled autograd traces the backward (the operators are its leaves): the same bits as the plain engine."""
+    import flare_b200 as fb
+    B, H, N, M, D = 2, 2, 150, 16, 16
+    g = torch.Generator().manual_seed(4)
+    x = [(torch.randn(*s, generator=g) * 0.5).bfloat16().to(cuda_dev).requires_grad_(True)
+         for s in ((H, M, D), (B, H, N, D), (B, H, M, D) if which == "scatter" else (B, H, N, D))]
+    if which == "autocast":
+        x[0] = x[0].detach().float().requires_grad_(True)
+    mask = (torch.arange(N, device=cuda_dev) < 100).expand(B, N) if which == "masked" else None
+
+    def loss():
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=which == "autocast"):
+            y = (fb.flare_gather(*x)[0] if which == "gather" else fb.flare_scatter(*x) if which == "scatter"
+                 else fb.flare_multihead_mixer(*x, key_mask=mask))
+        return y.float().square().sum()
+
+    want = torch.autograd.grad(loss(), x)
+    torch._dynamo.reset()
+    out = loss()
+    with torch._dynamo.compiled_autograd._enable(torch.compile(backend="eager")):
+        out.backward()
+    for t, w in zip(x, want):
+        assert torch.equal(t.grad, w)
