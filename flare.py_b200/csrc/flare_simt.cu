@@ -9,6 +9,7 @@
 //     latents in registers (scatter, dK/dV);     grid = (N-block, h, b).
 // Scores are kept in log2 units (scale*log2(e) folded into q) so that every
 // exponential is one ex2.
+#include <cfloat>
 #include "common.cuh"
 #include "launch.h"
 
@@ -758,7 +759,8 @@ k_scatter_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const fl
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     zero_row<D>(kr[r]); zero_row<D>(acc[r]);
-    mx[r] = -INFINITY; l[r] = 0.f;
+    // the lowest number and not -inf: a warp whose latents all score -inf then gives them weight 0 (-inf less -inf is NaN)
+    mx[r] = -FLT_MAX; l[r] = 0.f;
     const int tok = blockIdx.x * TPB + 32 * r + lane;
     if (tok < c.N) row_from_global<T, D>(kr[r], k + b * c.ks[0] + h * c.ks[1] + (long long)tok * c.ks[2], 1.f);
   }
@@ -822,7 +824,7 @@ k_scatter_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const fl
   __syncthreads();
   const int tok = blockIdx.x * TPB + threadIdx.x;
   if (threadIdx.x < TPB && tok < c.N) {
-    float m = -INFINITY;
+    float m = -FLT_MAX;
 #pragma unroll
     for (int w = 0; w < 4; ++w) m = fmaxf(m, sm[(w * TPB + threadIdx.x) * W + D]);
     float tot[D], ls = 0.f;
@@ -831,7 +833,7 @@ k_scatter_rows(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const fl
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const float* o = sm + (w * TPB + threadIdx.x) * W;
-      const float e = o[D] == -INFINITY ? 0.f : exp2f(o[D] - m);      // a warp without latents
+      const float e = exp2f(o[D] - m);             // (a warp without latents holds zeros)
 #pragma unroll
       for (int i = 0; i < D; ++i) tot[i] = fmaf(e, o[i], tot[i]);
       ls = fmaf(e, o[D + 1], ls);

@@ -513,3 +513,23 @@ def test_backward_under_compiled_autograd(cuda_dev, which):
         out.backward()
     for t, w in zip(x, want):
         assert torch.equal(t.grad, w)
+
+
+@pytest.mark.parametrize("D", [8, 16, 32])
+@pytest.mark.parametrize("N,H", [(40, 1), (5000, 8)])
+def test_scatter_with_scores_of_minus_infinity(cuda_dev, D, N, H):
+    """Latents whose scores overflow to -inf have weight 0, also where they fill the whole quarter of the latents that one
+    warp takes (128 latents in tiles of 2048 / D: the quarters begin at 0, 32, 64, 96 or at multiples of 16)."""
+    import flare_b200 as fb
+    M = 128
+    g = torch.Generator().manual_seed(6)
+    q = torch.randn(H, M, D, generator=g) * 1e-20
+    q[:, 32:] = -1e20
+    q[:, 70] = 1e-20
+    k = (torch.rand(1, H, N, D, generator=g) + 0.5) * 1e20
+    z = torch.randn(1, H, M, D, generator=g)
+    assert (q[0, 40] * k[0, 0, 0]).sum() == -float("inf")
+    y = fb.flare_scatter(q.to(cuda_dev), k.to(cuda_dev), z.to(cuda_dev))
+    want = O.scatter(q.double(), k.double(), z.double(), 1.0)
+    want = want[0] if isinstance(want, tuple) else want
+    assert O.rel_l2(y.double().cpu(), want) <= 1e-5
