@@ -265,7 +265,7 @@ def flare_multihead_mixer(q, k, v, scale: float = 1.0, key_mask: Optional[torch.
             k, v = _autocast(k, v)
         if q.dtype != dt and (q.dtype != torch.float32 or torch.compiler.is_compiling()):
             q, = _autocast(q)
-        if k.dtype != v.dtype:
+        if k.dtype != v.dtype or (q.dtype != k.dtype and (q.dtype != torch.float32 or k.dtype != dt)):
             _same_dtype(q, k, v)
     elif not q.dtype == k.dtype == v.dtype:
         _same_dtype(q, k, v)

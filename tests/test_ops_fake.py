@@ -112,3 +112,15 @@ def test_triple_attention_refuses_mismatched_sizes_before_any_launch(which, shap
     with FakeTensorMode():
         with pytest.raises(ValueError):
             fb.triple_attention(*(torch.empty(s, dtype=torch.float16, device="cuda") for s in shapes))
+
+
+@pytest.mark.parametrize("q_dtype,kv_dtype", [(torch.int32, torch.bfloat16), (torch.bool, torch.bfloat16), (torch.int64, torch.float32),
+                                             (torch.float32, torch.int32)])
+def test_latents_that_autocast_does_not_cast_are_refused(monkeypatch, q_dtype, kv_dtype):
+    """Autocast casts floating inputs only: integer latents do not meet 16-bit keys, nor the other way round."""
+    monkeypatch.setattr(torch, "is_autocast_enabled", lambda *a: True)
+    monkeypatch.setattr(torch, "get_autocast_dtype", lambda *a: torch.bfloat16)
+    with FakeTensorMode():
+        k = torch.empty(1, 2, 64, 16, device="cuda", dtype=kv_dtype)
+        with pytest.raises(TypeError):
+            fb.flare_multihead_mixer(torch.empty(2, 8, 16, device="cuda", dtype=q_dtype), k, k)
