@@ -27,15 +27,15 @@ def causal_state_init(B: int, H: int, M: int, D: int, device) -> torch.Tensor:
 
 def flare_causal_prefill(q, k, v, scale: float = 1.0, state=None):
     """All tokens of k, v [B,H,N,D] at once.  Returns (y [B,H,N,D], state after the last token)."""
-    return native.causal_prefill(q, k, v, scale, state)
+    return native.causal_prefill(q, k, v, float(scale), state)
 
 
 def flare_causal_decode(q, k, v, state, scale: float = 1.0):
     """The tokens of k, v [B,H,T,D] (T is usually 1) one after the other; `state` is updated in place."""
-    return native.causal_decode(q, k, v, state, scale)
+    return native.causal_decode(q, k, v, state, float(scale))
 
 
 def flare_causal_mixer(q, k, v, scale: float = 1.0):
     """Causal FLARE over a whole sequence, differentiable in q, k, v: token t sees the latent summary of
     tokens 0..t only.  q [H,M,D] (or [B,H,M,D]), k, v [B,H,N,D]; returns y [B,H,N,D]."""
-    return native.causal_mixer(q, k, v, scale)
+    return native.causal_mixer(q, k, v, float(scale))

@@ -106,46 +106,51 @@ def make_problem(q, k, scale: float, n_splits: int = 0, v=None, y=None, dy=None,
     return p
 
 
+def _seed64(seed) -> int:
+    """Any integer seed as the operator's signed 64 bits (the kernels see it modulo 2^64)."""
+    return ((int(seed) + (1 << 63)) & 0xFFFFFFFFFFFFFFFF) - (1 << 63)
+
+
 def mixer_forward(q, k, v, scale=1.0, key_mask=None, dropout_p=0.0, dropout_seed=0):
     """y, z32[B,H,M,D], lse_m[B,H,M], lse_n[B,H,N] via flare_mixer_fwd; not recorded by autograd."""
     _need_cuda(q, k, v)
     if not (q.dtype == k.dtype == v.dtype):
         raise TypeError("q, k, v must share a dtype")
     with torch.no_grad():
-        return ops.mixer_fwd(q, k, v, scale, key_mask, dropout_p, dropout_seed)
+        return ops.mixer_fwd(q, k, v, float(scale), key_mask, float(dropout_p), _seed64(dropout_seed))
 
 
 def mixer_backward(q, k, v, dy, y, z32, lse_m, lse_n, scale=1.0, key_mask=None, dropout_p=0.0, dropout_seed=0):
     """dq (fp32, [H,M,D] or [B,H,M,D]), dk, dv via flare_mixer_bwd."""
     _need_cuda(q, k, v, dy, y)
     with torch.no_grad():
-        return ops.mixer_bwd(q, k, v, dy, y, z32, lse_m, lse_n, scale, key_mask, dropout_p, dropout_seed)
+        return ops.mixer_bwd(q, k, v, dy, y, z32, lse_m, lse_n, float(scale), key_mask, float(dropout_p), _seed64(dropout_seed))
 
 
 def gather_forward(q, k, v, scale=1.0, key_mask=None):
     """z (input dtype), z32, lse_m[B,H,M] via flare_gather_partial + flare_combine; not recorded by autograd."""
     _need_cuda(q, k, v)
     with torch.no_grad():
-        return ops.gather_fwd(q, k, v, scale, key_mask)
+        return ops.gather_fwd(q, k, v, float(scale), key_mask)
 
 
 def gather_backward(q, k, v, dz, z32, lse_m, scale=1.0, key_mask=None):
     """dq (fp32), dk, dv of the gather alone (term 1 of the backward)."""
     with torch.no_grad():
-        return ops.gather_bwd(q, k, v, dz, z32, lse_m, scale, key_mask)
+        return ops.gather_bwd(q, k, v, dz, z32, lse_m, float(scale), key_mask)
 
 
 def scatter_forward(q, k, z, scale=1.0, key_mask=None):
     """y, lse_n[B,H,N] via flare_scatter; not recorded by autograd."""
     _need_cuda(q, k, z)
     with torch.no_grad():
-        return ops.scatter_fwd(q, k, z, scale, key_mask)
+        return ops.scatter_fwd(q, k, z, float(scale), key_mask)
 
 
 def scatter_backward(q, k, z, dy, y, lse_n, scale=1.0, key_mask=None):
     """dq (fp32), dk, dz (fp32) of the scatter alone (term 2 of the backward)."""
     with torch.no_grad():
-        return ops.scatter_bwd(q, k, z, dy, y, lse_n, scale, key_mask)
+        return ops.scatter_bwd(q, k, z, dy, y, lse_n, float(scale), key_mask)
 
 
 # ------------------------------------------------------------------------------------
@@ -279,7 +284,7 @@ def flare_multihead_mixer(q, k, v, scale: float = 1.0, key_mask: Optional[torch.
     if torch.compiler.is_compiling():
         _need_cuda(q, k, v)
         return ops.mixer_fwd(q, k, v, float(scale), key_mask, float(dropout_p), seed)[0]
-    return native.mixer(q, k, v, scale, key_mask, dropout_p, seed)
+    return native.mixer(q, k, v, float(scale), key_mask, float(dropout_p), seed)
 
 
 def flare_gather(q, k, v, scale: float = 1.0, key_mask=None):

@@ -124,3 +124,21 @@ def test_latents_that_autocast_does_not_cast_are_refused(monkeypatch, q_dtype, k
         k = torch.empty(1, 2, 64, 16, device="cuda", dtype=kv_dtype)
         with pytest.raises(TypeError):
             fb.flare_multihead_mixer(torch.empty(2, 8, 16, device="cuda", dtype=q_dtype), k, k)
+
+
+@pytest.mark.parametrize("seed", [0, -5, 2 ** 63 - 1, 2 ** 63 + 5, 2 ** 64 - 1, 2 ** 64 + 3])
+def test_dropout_seed_of_any_size_reaches_the_operator_modulo_2_64(seed):
+    got = []
+
+    class Record(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            got.append(args)
+            return func(*args, **(kwargs or {}))
+
+    with FakeTensorMode():
+        q, k = (torch.empty(s, device="cuda", dtype=torch.bfloat16) for s in ((2, 8, 16), (1, 2, 64, 16)))
+        with Record():
+            fb.mixer_forward(q, k, k, dropout_p=0.1, dropout_seed=seed)
+            fb.flare_multihead_mixer(q, k, k, "0.5")
+    assert got[0][6] % 2 ** 64 == seed % 2 ** 64
+    assert got[1][3] == 0.5                              # whatever float() takes is a scale
