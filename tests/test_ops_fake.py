@@ -132,7 +132,8 @@ def test_dropout_seed_of_any_size_reaches_the_operator_modulo_2_64(seed):
 
     class Record(TorchDispatchMode):
         def __torch_dispatch__(self, func, types, args=(), kwargs=None):
-            got.append(args)
+            if func is ops.mixer_fwd.default:
+                got.append(args)
             return func(*args, **(kwargs or {}))
 
     with FakeTensorMode():
