@@ -73,6 +73,7 @@ bool addressable(const Tensor& t) {
   const auto st = t.strides();
   const auto sz = t.sizes();
   const int64_t e = t.element_size(), nd = t.dim();
+  if (nd == 0) raise_py(PyExc_IndexError, "expected a tensor of four dimensions, got a scalar");
   if (st[nd - 1] != 1 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
   for (int64_t i = 0; i + 1 < nd; ++i)
     if ((st[i] * e) % 16 || (st[i] == 0 && sz[i] != 1)) return false;
@@ -105,6 +106,7 @@ Tensor scratch(size_t bytes, const Tensor& like) {
 }
 
 void set_stride(int64_t (&dst)[3], const Tensor& t) {
+  if (t.dim() < 3) raise_py(PyExc_ValueError, "expected a tensor of four dimensions, got " + std::to_string(t.dim()));
   const auto s = t.strides();
   for (int i = 0; i < 3; ++i) dst[i] = s[i];
 }

@@ -533,3 +533,17 @@ def test_scatter_with_scores_of_minus_infinity(cuda_dev, D, N, H):
     want = O.scatter(q.double(), k.double(), z.double(), 1.0)
     want = want[0] if isinstance(want, tuple) else want
     assert O.rel_l2(y.double().cpu(), want) <= 1e-5
+
+
+@pytest.mark.parametrize("which", ["mixer", "gather", "prefill", "decode", "causal", "linear"])
+def test_operands_of_too_few_dimensions_are_refused(cuda_dev, which):
+    """The refusal is the host's: the strides of a v of two dimensions are never read, and nothing is launched."""
+    import flare_b200 as fb
+    q, k, v = (torch.zeros(s, device=cuda_dev) for s in ((2, 16, 32), (1, 2, 64, 32), (64, 32)))
+    st = torch.zeros(1, 2, 16, 34, device=cuda_dev)
+    call = {"mixer": lambda: fb.flare_multihead_mixer(q, k, v), "gather": lambda: fb.flare_gather(q, k, v),
+            "prefill": lambda: fb.flare_causal_prefill(q, k, v), "decode": lambda: fb.flare_causal_decode(q, k, v, st),
+            "causal": lambda: fb.flare_causal_mixer(q.requires_grad_(True), k, v),
+            "linear": lambda: fb.causal_linear(v, k, k)}[which]
+    with pytest.raises(ValueError, match="dimensions"):
+        call()
