@@ -376,7 +376,7 @@ class ScatterFn : public torch::autograd::Function<ScatterFn> {
 
 Four mixer_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const optional<Tensor>& key_mask,
                         double dropout_p, int64_t dropout_seed) {
-  if (!at::GradMode::is_enabled() || !(q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+  if (!torch::autograd::compute_requires_grad(q, k, v)) {
     at::AutoDispatchBelowADInplaceOrView below;
     return Op_mixer_fwd::get().call(q, k, v, scale, key_mask, dropout_p, dropout_seed);
   }
@@ -423,10 +423,18 @@ Three scatter_bwd_autograd(const Tensor& q, const Tensor& k, const Tensor& z, co
   return no_second_derivative("flare_b200::scatter_bwd", std::move(r), q, k, z, dy, y, lse_n);
 }
 Three gather_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const optional<Tensor>& key_mask) {
+  if (!torch::autograd::compute_requires_grad(q, k, v)) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return Op_gather_fwd::get().call(q, k, v, scale, key_mask);
+  }
   auto r = GatherFn::apply(q, k, v, scale, key_mask);
   return {r[0], r[1], r[2]};
 }
 Two scatter_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& z, double scale, const optional<Tensor>& key_mask) {
+  if (!torch::autograd::compute_requires_grad(q, k, z)) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return Op_scatter_fwd::get().call(q, k, z, scale, key_mask);
+  }
   auto r = ScatterFn::apply(q, k, z, scale, key_mask);
   return {r[0], r[1]};
 }

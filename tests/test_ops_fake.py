@@ -143,3 +143,15 @@ def test_dropout_seed_of_any_size_reaches_the_operator_modulo_2_64(seed):
             fb.flare_multihead_mixer(q, k, k, "0.5")
     assert got[0][6] % 2 ** 64 == seed % 2 ** 64
     assert got[1][3] == 0.5                              # whatever float() takes is a scale
+
+
+def test_gather_and_scatter_take_forward_mode_inputs():
+    """As the mixer: a call that records no backward runs on the values of dual tensors (it makes no tangent)."""
+    import torch.autograd.forward_ad as fw
+    with FakeTensorMode():
+        q, k = torch.empty(2, 8, 16, device="cuda"), torch.empty(1, 2, 64, 16, device="cuda")
+        z = torch.empty(1, 2, 8, 16, device="cuda")
+        with fw.dual_level():
+            d = fw.make_dual(k, torch.ones_like(k))
+            assert fb.flare_gather(q, d, k)[0].shape == z.shape
+            assert fb.flare_scatter(q, d, z).shape == k.shape
