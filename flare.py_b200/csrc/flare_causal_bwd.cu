@@ -483,7 +483,8 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int chunks = (p->N + kChunk - 1) / kChunk;
   const long long rows = (long long)p->B * p->H * M;
-  if (causal_bwd_tc_supported(p, q, k, v, dy, dk, dv)) {
+  // (its last pass writes dq32 four values at a time; the fp32 kernel takes any float pointer)
+  if (causal_bwd_tc_supported(p, q, k, v, dy, dk, dv) && reinterpret_cast<uintptr_t>(dq32) % 16 == 0) {
     // one chunk per CTA on the tensor cores, behind the forward's record and scan passes
     const Prefix pre(p, workspace);
     int rc = causal_tc_prefix(p, q, k, v, pre.pacc, pre.plo, pre.pml, nullptr, nullptr, chunks, st);
@@ -528,6 +529,7 @@ int flare_causal_train_bwd(const FlareProblem* p, const void* q, const void* k, 
   const int ok = check_args(p, q, k, v, dy, dq32, dk, dv, workspace);
   if (ok != FLARE_OK) return ok;
   if (!saved) return refuse(FLARE_EINVAL, "causal_train_bwd: null pointer");
+  if (reinterpret_cast<uintptr_t>(dq32) % 16) return refuse(FLARE_EALIGN, "causal_train_bwd: dq32 must be 16-byte aligned");
   if (!causal_bwd_tc_supported(p, q, k, v, dy, dk, dv))
     return refuse(FLARE_EUNSUPPORTED, "causal_train_bwd: bf16, M <= 128, D in {32,64}, 16-byte aligned rows only");
   const Prefix pre(p, const_cast<void*>(saved));

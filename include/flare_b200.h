@@ -270,7 +270,8 @@ int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const 
 
 /* The training pair of the tensor-core shapes: the forward leaves the chunk-start states in `saved`
  * (flare_causal_train_bytes(p) bytes, 0 for a shape these two do not serve) and the backward starts from them instead
- * of rebuilding them.  dq32 is fp32 [H][M][D], summed over the batch, when q_stride[0] == 0, else [B][H][M][D]. */
+ * of rebuilding them.  dq32 is fp32 [H][M][D], summed over the batch, when q_stride[0] == 0, else [B][H][M][D];
+ * 16-byte aligned. */
 size_t flare_causal_train_bytes(const FlareProblem* p);
 size_t flare_causal_train_bwd_workspace_bytes(const FlareProblem* p);
 int flare_causal_train_fwd(const FlareProblem* p, const void* q, const void* k, const void* v, void* y, void* saved,

@@ -110,6 +110,16 @@ def test_causal_prefill_workspace_size_and_alignment_are_host_checks(cabi):
     assert b"aligned" in cabi.lib.flare_last_error()
 
 
+def test_causal_train_backward_refuses_a_misaligned_latent_gradient(cabi):
+    """Its last pass stores dq32 in pieces of 16 bytes: any other pointer is refused before any launch."""
+    p = _problem(cabi, N=1000, M=64, D=32, dtype=cabi.BF16)
+    for f in ("q_stride", "k_stride", "v_stride", "dy_stride", "dk_stride", "dv_stride"):
+        getattr(p, f)[:] = (8 * 1000 * 32, 1000 * 32, 32)
+    for off in (4, 8, 12):
+        rc = cabi.lib.flare_causal_train_bwd(C.byref(p), 16, 16, 16, 16, 16, 16 + off, 16, 16, 256, None)
+        assert rc == -2 and b"dq32" in cabi.lib.flare_last_error()
+
+
 def test_whole_pass_checks_workspace(cabi):
     p = _problem(cabi)
     rc = cabi.lib.flare_mixer_fwd(C.byref(p), 16, 16, 16, None, 16, 16, 16, 16, 256, 8, None)

@@ -287,6 +287,27 @@ def test_backward_hands_wide_heads_to_the_fp32_kernel(cuda_dev):
             assert O.rel_l2(g.double().cpu(), r) <= 5e-3, h
 
 
+def test_c_backward_takes_any_float_pointer_for_the_latent_gradient(cuda_dev):
+    """flare_causal_bwd with dq32 at 4 bytes past a 16-byte boundary: the fp32 kernel takes it.  Both forms start from
+    16-bit records (below 1e-3 of the fp64 gradient), so they agree to twice that."""
+    import ctypes as C
+    fb = _fb()
+    from flare_b200 import _cabi
+    from flare_b200.mixer import make_problem
+    B, H, N, M, D = 1, 2, 300, 64, 32
+    q, k, v, dy = (t.to(cuda_dev) for t in O.make_inputs(B, H, N, M, D, dtype=torch.bfloat16, seed=35))
+    got = []
+    for off in (0, 1):
+        dk, dv, buf = torch.empty_like(k), torch.empty_like(v), torch.zeros(B * H * M * D + 4, device=cuda_dev)
+        dq = buf[off:off + B * H * M * D]
+        p = make_problem(q, k, 1.0, v=v, dy=dy, dk=dk, dv=dv)
+        ws = torch.empty(_cabi.lib.flare_causal_bwd_workspace_bytes(C.byref(p)), dtype=torch.uint8, device=cuda_dev)
+        _cabi.check(_cabi.lib.flare_causal_bwd(C.byref(p), *(_cabi.ptr(t) for t in (q, k, v, dy, dq, dk, dv, ws)), _cabi.stream_of(q)), "bwd")
+        got.append(dq.clone())
+    assert fb.device_status() == 0
+    assert O.rel_l2(got[1], got[0]) <= 2e-3
+
+
 def test_mixer_without_gradients_is_the_plain_prefill(cuda_dev):
     """No gradient wanted: the kernels of the prefill, to the bit (the training forward keeps its chunk prefixes in two terms)."""
     fb = _fb()
