@@ -3,6 +3,8 @@
 The reference has no code for this path, so the oracle itself is checked for self-consistency
 (tests/test_oracle.py); here the CUDA prefill and decode are compared with it.
 """
+import math
+
 import pytest
 import torch
 
@@ -241,7 +243,7 @@ def test_backward_long_sequence_against_the_chunked_restatement(cuda_dev, dtype,
     (1, 1, 129, 64, 64),       # a last chunk of one token, fewer latents than rows
     (1, 2, 5, 32, 32),
     (2, 1, 1000, 96, 32),      # a latent count that is no multiple of 64
-    (1, 64, 4800, 128, 32),    # 2432 chunks: two to a unit, units taken in several rounds
+    (1, 64, 4800, 128, 32),    # 2432 chunks, one to a unit: every CTA takes sixteen or seventeen of them
 ])
 def test_backward_on_tensor_cores(cuda_dev, B, H, N, M, D):
     """bf16 with M <= 128 and D in {32, 64}: one chunk per CTA, the suffix state handed from chunk to chunk.
@@ -267,6 +269,20 @@ def test_backward_error_is_that_of_rounding_the_results(cuda_dev, N, M, D):
         assert O.rel_l2(t.grad.double().cpu(), r) < 1.85e-3, n
 
 
+def _too_wide(q, k, margin=5.0):
+    """Whether a head leaves the range of the tensor-core backward in some 128-token chunk: in octaves, a latent's maximum
+    climbing by more than 64 after the chunk's first token, or a row or column maximum more than 50 from that token's
+    column maximum.  A head within `margin` of a limit is neither."""
+    S, top, m0 = (q @ k.t()) / math.log(2.0), -math.inf, torch.full((q.shape[0],), -math.inf, dtype=q.dtype)
+    for c in range(0, k.shape[0], 128):
+        s = S[:, c:c + 128]
+        mu, first, cm = torch.maximum(m0, s.amax(1)), torch.maximum(m0, s[:, 0]), s.amax(0)
+        top = max(top, ((mu - first).max() - 64).item(), ((mu - cm[0]).abs().max() - 50).item(), ((cm - cm[0]).abs().max() - 50).item())
+        m0 = mu
+    assert abs(top) > margin
+    return top > 0
+
+
 def test_backward_hands_wide_heads_to_the_fp32_kernel(cuda_dev):
     """Scores that climb past 64 octaves inside a chunk in one of three heads: that head is redone by the fp32
     kernel (finite, same tolerance), the others stay as they are."""
@@ -275,6 +291,7 @@ def test_backward_hands_wide_heads_to_the_fp32_kernel(cuda_dev):
     q, k, v, dy = O.make_inputs(B, H, N, M, D, dtype=torch.bfloat16, seed=29)
     k = k.clone()
     k[:, 1, 128:256] = (k[:, 1, 128:256].float() * torch.linspace(0.1, 40.0, 128).view(1, 128, 1)).bfloat16()
+    assert [_too_wide(q[h].double(), k[0, h].double()) for h in range(H)] == [False, True, False]
     qd, kd, vd = (t.to(cuda_dev).requires_grad_(True) for t in (q, k, v))
     y = fb.flare_causal_mixer(qd, kd, vd, 1.0)
     y.backward(dy.to(cuda_dev))
