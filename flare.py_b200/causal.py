@@ -37,5 +37,10 @@ def flare_causal_decode(q, k, v, state, scale: float = 1.0):
 
 def flare_causal_mixer(q, k, v, scale: float = 1.0):
     """Causal FLARE over a whole sequence, differentiable in q, k, v: token t sees the latent summary of
-    tokens 0..t only.  q [H,M,D] (or [B,H,M,D]), k, v [B,H,N,D]; returns y [B,H,N,D]."""
+    tokens 0..t only.  q [H,M,D] (or [B,H,M,D]), k, v [B,H,N,D]; returns y [B,H,N,D].
+
+    Where a gradient is wanted, bf16 with M <= 128 and D in {32, 64} keeps the states before every 128-token chunk for
+    the backward: M (4 D + 8) bytes per chunk and head, next to q, k and v (138 MB at B = 4, H = 16, N = 8192, M = 128,
+    D = 64, where k and v are 134 MB).  They are ordinary saved tensors: torch.utils.checkpoint around the call rebuilds
+    them, torch.autograd.graph.save_on_cpu moves them away."""
     return native.causal_mixer(q, k, v, float(scale))

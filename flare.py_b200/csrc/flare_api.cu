@@ -51,8 +51,12 @@ int check_tok(const char* name, const void* ptr, const int64_t* st, int dtype) {
 // Estimated device time (microseconds) of the passes that run one CTA per (b, h, latent block, token range), for S ranges
 // of `tiles` 128-token tiles.  What decides is how full the last wave of CTAs is: 19 ranges for 8 heads are 152
 // one-per-SM CTAs of the backward, two waves where 18 ranges take one (1.86 -> 1.16 ms at N = 300 007, M = 512, D = 32).
-// Measured times per CTA and tile: latent-major passes 1.7 with two CTAs on the SM, 1.12 alone; one-exponential backward
-// 1.5, general backward 5.5 (per 128 latents); set-up 4 and 12 per CTA.
+// Times per CTA and tile as measured when the rule was made: latent-major passes 1.7 with two CTAs on the SM, 1.12 alone;
+// one-exponential backward 1.5, general backward 5.5 (per 128 latents); set-up 4 and 12 per CTA.  The general backward has
+// become faster since: at D = 16 3.9 alone and 5.0 with two CTAs on the SM (M = 128; M = 256: 3.3 and 4.4), at D = 32 3.8
+// (3.1).  So the rule gives it too much weight, and since it does not see the mask it counts every bf16 call of D = 32
+// as one-exponential, which masked and dropped-out ones are not.  Against the ranges of before it (four CTAs per SM in
+// flight, whatever they fill) none of 60 sizes timed, masked, dropped-out, fp16 and fp32 ones among them, takes longer.
 double split_cost(const FlareProblem* p, bool tc, long long tiles, long long S) {
   const long long bh = (long long)p->B * p->H, nb = (p->M + 127) / 128, per = (tiles + S - 1) / S;
   const double parts = (double)S * bh * p->M * (p->D + 2) * 4 * 3 / 2.5e6;          // partial records written and read again

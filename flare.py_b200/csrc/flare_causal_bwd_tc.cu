@@ -23,12 +23,14 @@
 // Operands.  Every 128 x 128 operand is written where the next product reads it: rows of E, G, dS packed in tensor
 // memory (A operand, contraction over the tokens) and as 64-token column blocks in shared memory (MN-major operand,
 // contraction over the latents); X once, masked to t >= n, serves as the MN-major operand of C and the K-major operand
-// of de.  All of them, and a acc0, Rin and W, are carried as two bf16 terms (value and remainder), so that the
-// contractions see about 16 bits and the error of dq, dk, dv is that of rounding the results: with one term of E, G in
-// W and Gg, a acc0 and Rin they were 2.23e-3, 2.08e-3, 1.74e-3 off (B = 1, H = 8, N = 512, M = 128, D = 64; rounding
-// alone is 1.67e-3), now 1.72e-3, 1.71e-3, 1.68e-3, as in the fp32 kernel.  Shared memory has room for one pair of remainders at a time: first those
-// of E and G, for W; then X, which waits in tensor memory until W is complete; then dS.  The second term of E^T Rin comes
-// last, over E.
+// of de.  All of them, and a acc0, Rin and W, are carried as two bf16 terms (value and remainder; remainder times
+// remainder is dropped), about 16 bits where the fp32 kernel has 24: a chunk's own contractions are off by 4e-6 to 1e-5,
+// there by 1e-7 to 6e-7.  That is far below what both start from, chunk records with 16-bit weights: dq32 is 1.8e-4 to
+// 7.1e-4 off in both, the same to three or four digits (N from 200 to 8192, M = 64 and 128, D = 32 and 64, with wide heads
+// too), and dq, dk, dv after their rounding to bf16 (1.67e-3) as well.  With one term of E, G in W and Gg, a acc0 and Rin
+// they were 2.23e-3, 2.08e-3, 1.74e-3 off (B = 1, H = 8, N = 512, M = 128, D = 64) instead of 1.72e-3, 1.71e-3, 1.68e-3.
+// Shared memory has room for one pair of remainders at a time: first those of E and G, for W; then X, which waits in
+// tensor memory until W is complete; then dS.  The second term of E^T Rin comes last, over E.
 //
 // Tensor memory (512 columns):   0 S | E, G packed | G remainder over E | dS, dS remainder
 //                              128 S^T | W^T | W packed in place
@@ -37,9 +39,11 @@
 //
 // Range: E, l and G are relative to the chunk's final maximum, as in the forward walk, with the same bounds (64
 // octaves of climb, 50 between the latents' maxima and the first token's column maximum).  A (b, h) with a chunk
-// outside them is flagged and redone by the fp32 kernel behind this one.
+// outside them is flagged and redone as a whole by the fp32 kernel behind this one, from the same two-term prefixes.
+// That kernel walks a head alone: one flagged head at the shape below makes the step 20.5 ms (20.05 when it took them all).
 //
-// B = 4, H = 16, N = 8192, D = 64, M = 128: see the launcher for what was measured.
+// B = 4, H = 16, N = 8192, D = 64, M = 128: 546 us for 4096 chunks (the fp32 kernel: 19.1 ms), about 20 us a chunk, of which
+// the products are a small part: six waits for products a chunk and no second chunk on the SM to fill them.
 #include "common.cuh"
 #include "launch.h"
 #include "tc_common.cuh"

@@ -425,7 +425,7 @@ k_bwd_tokens(Ctx c, const T* __restrict__ q, const T* __restrict__ k, const T* _
 // R is what the registers hold: R * D * (operands + accumulators) <= 160 floats.  Measured, one row per thread against
 // these: N = 500 000, H = 8, M = 512, D = 8 bf16: gather 3.03 -> 1.82 ms, scatter 2.33 -> 1.89, dZ 2.93 -> 1.54, tokens
 // 7.23 -> 4.67, dQ 8.19 -> 4.47; B = 2, H = 8, N = 4096, M = 64, D = 16 fp32: dQ 98 -> 28 us, gather 36 -> 15, dZ 41 -> 16;
-// N = 5000, M = 64, D = 32 fp32: dQ 190 -> 96.  The token pass of D = 8 takes two rows, not four (250 registers: 4.80 ms).
+// N = 5000, M = 64, D = 32 fp32: dQ 190 -> 79.  The token pass of D = 8 takes two rows, not four (250 registers: 4.80 ms).
 // ---------------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ float dot2(const float2* a, const float2* b) {

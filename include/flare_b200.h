@@ -261,9 +261,10 @@ int flare_causal_decode(const FlareProblem* p, const void* q, const void* k, con
  * (b, h): sum over b when the latents are shared), dk, dv with dk_stride / dv_stride, from dy (dy_stride).
  * A reverse scan over 128-token chunks on the forward's own chunk-start records, which it rebuilds in
  * `workspace` (flare_causal_bwd_workspace_bytes(p) bytes).  D in {16,32,64}, M * D <= 8192.  bf16 with M <= 128,
- * D in {32,64} runs one chunk per CTA on the tensor cores; the other shapes, and any (b, h) whose scores span too many
- * octaves for that, one CTA per (b, h) in fp32 arithmetic.  No reference code exists for this path: the algorithm is checked against autograd
- * through the dense definition (oracle/flare_oracle.py: causal_bwd_chunked, causal_bwd_autograd). */
+ * D in {32,64} runs one chunk per CTA on the tensor cores (operands as two bf16 terms; dq32 16-byte aligned); the other
+ * shapes and pointers, and any (b, h) whose scores span too many octaves for that, one CTA per (b, h) in fp32
+ * arithmetic.  No reference code exists for this path: the algorithm is checked against autograd through the dense
+ * definition (oracle/flare_oracle.py: causal_bwd_chunked, causal_bwd_autograd). */
 size_t flare_causal_bwd_workspace_bytes(const FlareProblem* p);
 int flare_causal_bwd(const FlareProblem* p, const void* q, const void* k, const void* v, const void* dy,
                      float* dq32, void* dk, void* dv, float* workspace, flare_stream_t stream);

@@ -325,6 +325,23 @@ def test_c_backward_takes_any_float_pointer_for_the_latent_gradient(cuda_dev):
     assert O.rel_l2(got[1], got[0]) <= 2e-3
 
 
+@pytest.mark.parametrize("how", ["checkpoint", "save_on_cpu"])
+def test_kept_states_can_be_rebuilt_or_moved_away(cuda_dev, how):
+    """The chunk-start states of the training forward are ordinary saved tensors."""
+    from torch.utils.checkpoint import checkpoint
+    fb = _fb()
+    q, k, v, dy = (t.to(cuda_dev) for t in O.make_inputs(1, 4, 1000, 128, 64, dtype=torch.bfloat16, seed=36))
+    x = [t.requires_grad_(True) for t in (q, k, v)]
+    want = torch.autograd.grad(fb.flare_causal_mixer(*x, 1.0), x, dy)
+    if how == "checkpoint":
+        y = checkpoint(fb.flare_causal_mixer, *x, 1.0, use_reentrant=False)
+    else:
+        with torch.autograd.graph.save_on_cpu():
+            y = fb.flare_causal_mixer(*x, 1.0)
+    for a, b in zip(torch.autograd.grad(y, x, dy), want):
+        assert torch.equal(a, b)
+
+
 def test_mixer_without_gradients_is_the_plain_prefill(cuda_dev):
     """No gradient wanted: the kernels of the prefill, to the bit (the training forward keeps its chunk prefixes in two terms)."""
     fb = _fb()
