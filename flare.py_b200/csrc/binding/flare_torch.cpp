@@ -307,11 +307,14 @@ FLARE_OP(scatter_bwd)
 Tensor as_dtype(const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt ? t : t.to(dt); }
 optional<Tensor> maybe(const Tensor& t) { return t.defined() ? optional<Tensor>(t) : std::nullopt; }
 
+// The autograd functions of the operators return the result alone; z32 and the log-sum-exps, the backward's operands and not
+// results anyone differentiates, reach the caller through `rest`.  As outputs they would have to be marked as
+// non-differentiable, which compiled autograd refuses, or be wrapped and saved as differentiable ones (6 us a step).
 class MixerFn : public torch::autograd::Function<MixerFn> {
  public:
   static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
-  static variable_list forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k, const Tensor& v, double scale,
-                               const optional<Tensor>& key_mask, double dropout_p, int64_t dropout_seed) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k, const Tensor& v, double scale,
+                        const optional<Tensor>& key_mask, double dropout_p, int64_t dropout_seed, Three* rest) {
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor q = as_dtype(q_, k.scalar_type());
     auto [y, z32, lse_m, lse_n] = Op_mixer_fwd::get().call(q, k, v, scale, key_mask, dropout_p, dropout_seed);
@@ -320,57 +323,58 @@ class MixerFn : public torch::autograd::Function<MixerFn> {
     ctx->saved_data["p"] = dropout_p;
     ctx->saved_data["seed"] = dropout_seed;
     ctx->saved_data["qdt"] = (int64_t)q_.scalar_type();
-    // z32, lse_m, lse_n are the backward's operands, not results anyone differentiates: no zero gradients for them (compiled
-    // autograd refuses a function that marks outputs as non-differentiable)
     ctx->set_materialize_grads(false);
-    return {y, z32, lse_m, lse_n};
+    *rest = {z32, lse_m, lse_n};
+    return y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-    if (!g[0].defined()) return variable_list(7);
+    if (!g[0].defined()) return variable_list(8);
     const auto s = ctx->get_saved_variables();
     auto [dq, dk, dv] = Op_mixer_bwd::get().call(s[0], s[1], s[2], g[0], s[3], s[4], s[5], s[6], ctx->saved_data["scale"].toDouble(),
                                                  maybe(s[7]), ctx->saved_data["p"].toDouble(), ctx->saved_data["seed"].toInt());
-    return {as_dtype(dq, (at::ScalarType)ctx->saved_data["qdt"].toInt()), dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+    return {as_dtype(dq, (at::ScalarType)ctx->saved_data["qdt"].toInt()), dk, dv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
 class GatherFn : public torch::autograd::Function<GatherFn> {
  public:
   static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
-  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale,
-                               const optional<Tensor>& key_mask) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale,
+                        const optional<Tensor>& key_mask, Two* rest) {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [z, z32, lse_m] = Op_gather_fwd::get().call(q, k, v, scale, key_mask);
     ctx->save_for_backward({q, k, v, z32, lse_m, key_mask.value_or(Tensor())});
     ctx->saved_data["scale"] = scale;
     ctx->set_materialize_grads(false);
-    return {z, z32, lse_m};
+    *rest = {z32, lse_m};
+    return z;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-    if (!g[0].defined()) return variable_list(5);
+    if (!g[0].defined()) return variable_list(6);
     const auto s = ctx->get_saved_variables();
     auto [dq, dk, dv] = Op_gather_bwd::get().call(s[0], s[1], s[2], g[0], s[3], s[4], ctx->saved_data["scale"].toDouble(), maybe(s[5]));
-    return {as_dtype(dq, s[0].scalar_type()), dk, dv, Tensor(), Tensor()};
+    return {as_dtype(dq, s[0].scalar_type()), dk, dv, Tensor(), Tensor(), Tensor()};
   }
 };
 
 class ScatterFn : public torch::autograd::Function<ScatterFn> {
  public:
   static constexpr bool is_traceable = true;       // compiled autograd may trace the backward: it calls operators only
-  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& z, double scale,
-                               const optional<Tensor>& key_mask) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& z, double scale,
+                        const optional<Tensor>& key_mask, Tensor* rest) {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [y, lse_n] = Op_scatter_fwd::get().call(q, k, z, scale, key_mask);
     ctx->save_for_backward({q, k, z, y, lse_n, key_mask.value_or(Tensor())});
     ctx->saved_data["scale"] = scale;
     ctx->set_materialize_grads(false);
-    return {y, lse_n};
+    *rest = lse_n;
+    return y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-    if (!g[0].defined()) return variable_list(5);
+    if (!g[0].defined()) return variable_list(6);
     const auto s = ctx->get_saved_variables();
     auto [dq, dk, dz] = Op_scatter_bwd::get().call(s[0], s[1], s[2], g[0], s[3], s[4], ctx->saved_data["scale"].toDouble(), maybe(s[5]));
-    return {as_dtype(dq, s[0].scalar_type()), dk, as_dtype(dz, s[2].scalar_type()), Tensor(), Tensor()};
+    return {as_dtype(dq, s[0].scalar_type()), dk, as_dtype(dz, s[2].scalar_type()), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -380,8 +384,9 @@ Four mixer_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, doubl
     at::AutoDispatchBelowADInplaceOrView below;
     return Op_mixer_fwd::get().call(q, k, v, scale, key_mask, dropout_p, dropout_seed);
   }
-  auto r = MixerFn::apply(q, k, v, scale, key_mask, dropout_p, dropout_seed);
-  return {r[0], r[1], r[2], r[3]};
+  Three rest;
+  const Tensor y = MixerFn::apply(q, k, v, scale, key_mask, dropout_p, dropout_seed, &rest);
+  return {y, std::get<0>(rest), std::get<1>(rest), std::get<2>(rest)};
 }
 // The backward operators have no derivative of their own: where a graph of them is recorded (create_graph), differentiating
 // their results raises instead of leaving their share out.
@@ -427,16 +432,18 @@ Three gather_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, dou
     at::AutoDispatchBelowADInplaceOrView below;
     return Op_gather_fwd::get().call(q, k, v, scale, key_mask);
   }
-  auto r = GatherFn::apply(q, k, v, scale, key_mask);
-  return {r[0], r[1], r[2]};
+  Two rest;
+  const Tensor z = GatherFn::apply(q, k, v, scale, key_mask, &rest);
+  return {z, std::get<0>(rest), std::get<1>(rest)};
 }
 Two scatter_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& z, double scale, const optional<Tensor>& key_mask) {
   if (!torch::autograd::compute_requires_grad(q, k, z)) {
     at::AutoDispatchBelowADInplaceOrView below;
     return Op_scatter_fwd::get().call(q, k, z, scale, key_mask);
   }
-  auto r = ScatterFn::apply(q, k, z, scale, key_mask);
-  return {r[0], r[1]};
+  Tensor lse_n;
+  const Tensor y = ScatterFn::apply(q, k, z, scale, key_mask, &lse_n);
+  return {y, lse_n};
 }
 
 // ------------------------------------------------------------------------------------------------
